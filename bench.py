@@ -52,7 +52,7 @@ import numpy as np  # noqa: E402
 WORKLOAD = dict(workload="spheres-1m", scene="spheres-1m", triangles=1310978, width=1920, height=1080, spp=64,
                 depth=12, nee=True, lights=256, pool=1 << 20)
 TRACE_ALGO_BYTES_PER_RAY = 32 + 48   # ray record read, material-queue entry (ray and hit) written; a miss writes none
-NODE_BYTES = 64 + 4   # a BVH8 node visit reads the 64-byte header (boxes, origin, scales, masks) and its 4-byte reference
+NODE_BYTES = 64       # a BVH8 node visit reads the 64-byte header (boxes, origin, scales, child block)
 TRIANGLE_BYTES = 48
 
 

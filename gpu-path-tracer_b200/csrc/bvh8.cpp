@@ -20,7 +20,7 @@
 //  4. Child boxes are padded (1e-5 of their largest extent, plus a relative 1e-7 of their
 //     coordinates) and quantised to 8 bits per axis against the node origin with a power-of-two
 //     scale, rounding outward; every quantised box is checked in exact arithmetic to contain the
-//     padded child box.
+//     padded child box. The origin is a 24-bit multiple of a power of two.
 #include "bvh8.hpp"
 
 #include <algorithm>
@@ -492,14 +492,56 @@ namespace pt
         };
 
         // Wide nodes in depth-first pre-order (a node, then the subtrees of its inner children in slot
-        // assignment order). Every subtree's place is known from the plan's node counts, so large
-        // subtrees are written by other threads into their own ranges of the preallocated array.
+        // assignment order); node j's children are block j + 1. Every subtree's place is known from the
+        // plan's node counts, so large subtrees are written by other threads into their own ranges of
+        // the preallocated array.
         struct WideBuilder
         {
             const BinaryBuilder& bin;
             CollapsePlan& plan;
-            std::vector<Node8> out;
+            const uint32_t* models;
+            std::vector<Record8> out;
+            std::vector<uint32_t> masks;
+            std::vector<uint32_t> leafRecord;    // by first leaf position: the record of a binary leaf's first triangle
+            std::atomic<uint32_t> nextExtra{0};  // record of the next further triangle of a leaf
             std::atomic<uint32_t> maxDepth{0};
+
+            void prepare(uint32_t nodes, uint32_t binaryNodes)
+            {
+                // a full binary tree of B nodes has (B + 1) / 2 leaves; further triangles of a leaf go behind the nodes' blocks
+                const uint32_t extra = bin.n - (binaryNodes + 1) / 2;
+                const size_t blocks = static_cast<size_t>(nodes) + 1 + (extra + kBlockRecords - 1) / kBlockRecords;
+                if (blocks > kMaxBlocks) throw std::runtime_error("BVH8 has more than 2^24 nodes");
+                out.resize(blocks * kBlockRecords);
+                masks.assign(blocks, 0u);
+                leafRecord.assign(bin.n, 0u);
+                nextExtra = (nodes + 1) * kBlockRecords;
+                for (uint32_t k = 0; k < extra; k++) masks[nodes + 1 + k / kBlockRecords] |= block_mask(0u, 1u << (k % kBlockRecords));
+                masks[0] = block_mask(1u, 0u);  // the root's header
+            }
+
+            // The triangles of a leaf, the first one in `record`.
+            void emit_leaf(const BNode& leaf, uint32_t record)
+            {
+                if (leaf.count > 255) throw std::runtime_error("BVH leaf larger than 255 triangles");
+                leafRecord[leaf.first] = record;
+                uint32_t extra = leaf.count > 1 ? nextExtra.fetch_add(leaf.count - 1) : 0u;
+                for (uint32_t j = 0; j < leaf.count; j++)
+                {
+                    const uint32_t t = bin.idx[leaf.first + j];
+                    const uint32_t next = j + 1 < leaf.count ? extra++ : 0u;
+                    const float* p = bin.pos + static_cast<size_t>(t) * 9;
+                    const float e[6] = {p[3] - p[0], p[4] - p[1], p[5] - p[2], p[6] - p[0], p[7] - p[1], p[8] - p[2]};
+                    uint32_t v[3], d[6];
+                    std::memcpy(v, p, sizeof(v));
+                    std::memcpy(d, e, sizeof(d));
+                    Record8& r = out[record];
+                    r.w[0] = make_uint4(v[0], v[1], v[2], t);
+                    r.w[1] = make_uint4(d[0], d[1], d[2], models[t]);
+                    r.w[2] = make_uint4(d[3], d[4], d[5], next);
+                    record = next;
+                }
+            }
 
             static void padBox(const Box& in, double lo[3], double hi[3])
             {
@@ -517,7 +559,8 @@ namespace pt
                 }
             }
 
-            void emit(uint32_t bnode, uint32_t depth, uint32_t me)
+            // Wide node `me` of binary node bnode; its header goes into `record`.
+            void emit(uint32_t bnode, uint32_t depth, uint32_t me, uint32_t record)
             {
                 uint32_t seen = maxDepth.load();
                 while (seen < depth + 1 && !maxDepth.compare_exchange_weak(seen, depth + 1)) {}
@@ -559,32 +602,29 @@ namespace pt
                     slotUsed[bs] = true;
                     slotOf[bk] = bs;
                 }
-                // child references: inner children's subtrees follow this node in the order of the children list
-                uint32_t childRef[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                uint8_t counts[8] = {};
-                uint8_t innerMask = 0, leafMask = 0;
+                // the children's block; inner children's subtrees follow this node in the order of the children list
+                const uint32_t block = me + 1;
+                uint32_t innerMask = 0, leafMask = 0;
                 uint32_t next = me + 1;
                 std::vector<std::future<void>> futs;
                 for (size_t i = 0; i < kids.size(); i++)
                 {
                     const BNode& c = bin.nodes[kids[i]];
                     const int s = slotOf[i];
+                    const uint32_t child = block * kBlockRecords + static_cast<uint32_t>(s);
                     if (kidLeaf[i])
                     {
-                        if (c.count > 255) throw std::runtime_error("BVH leaf larger than 255 triangles");
-                        childRef[s] = c.first | (c.count << 24);  // first triangle (24 bits), count (8 bits)
-                        counts[s] = static_cast<uint8_t>(c.count);
-                        leafMask |= static_cast<uint8_t>(1u << s);
+                        emit_leaf(c, child);
+                        leafMask |= 1u << s;
                     }
                     else
                     {
                         const uint32_t at = next, k = kids[i];
                         next += plan.wide[k];
-                        childRef[s] = at;
-                        innerMask |= static_cast<uint8_t>(1u << s);
+                        innerMask |= 1u << s;
                         std::future<void> fut;
-                        if (plan.spawn_if_free(c.count, [this, k, depth, at] { emit(k, depth + 1, at); }, fut)) futs.push_back(std::move(fut));
-                        else emit(k, depth + 1, at);
+                        if (plan.spawn_if_free(c.count, [this, k, depth, at, child] { emit(k, depth + 1, at, child); }, fut)) futs.push_back(std::move(fut));
+                        else emit(k, depth + 1, at, child);
                     }
                 }
                 for (auto& f : futs) f.get();
@@ -603,25 +643,38 @@ namespace pt
                         phi[a] = std::max(phi[a], chi[s][a]);
                     }
                 }
-                float p[3];
+                // origins: multiples of 2^unit that have 24 bits; scales within the header's range of the unit
+                int32_t origin[3];
                 int expo[3];
                 uint8_t qlo[3][8], qhi[3][8];
+                int unit = kMinUnit8;
                 for (int a = 0; a < 3; a++)
                 {
-                    // origin rounded down to float
-                    float pf = static_cast<float>(plo[a]);
-                    if (static_cast<double>(pf) > plo[a]) pf = std::nextafter(pf, -FLT_MAX);
-                    p[a] = pf;
-                    const double ext = phi[a] - static_cast<double>(pf);
-                    int e = -126;
+                    int fe;
+                    std::frexp(std::max(std::fabs(plo[a]), 1e-300), &fe);
+                    unit = std::max(unit, fe - 23);
+                }
+                for (int a = 0; a < 3;)
+                {
+                    const double grid = std::ldexp(1.0, unit);
+                    const double q0 = std::floor(plo[a] / grid);
+                    const double pf = q0 * grid;
+                    const double ext = phi[a] - pf;
+                    int e = unit - kScaleBelow8;
                     if (ext > 0.0)
                     {
                         int fe;
                         std::frexp(ext / 255.0, &fe);  // ext/255 = m * 2^fe, m in [0.5, 1)
-                        e = std::max(-126, std::min(127, fe));
+                        e = std::max(e, std::min(127, fe));
                     }
-                    for (;;)
+                    bool fits = std::fabs(q0) <= static_cast<double>(kMaxOrigin8);
+                    for (; fits; e++)
                     {
+                        if (e > unit + kScaleAbove8 || e > 127)
+                        {
+                            fits = false;
+                            break;
+                        }
                         const double scale = std::ldexp(1.0, e);
                         bool ok = true;
                         for (int s = 0; s < 8 && ok; s++)
@@ -635,28 +688,37 @@ namespace pt
                             double ql = std::floor((clo[s][a] - pf) / scale);
                             double qh = std::ceil((chi[s][a] - pf) / scale);
                             ql = std::max(0.0, ql);
-                            while (ql > 0 && static_cast<double>(pf) + ql * scale > clo[s][a]) ql -= 1.0;
-                            while (static_cast<double>(pf) + qh * scale < chi[s][a]) qh += 1.0;
-                            if (qh > 255.0 || static_cast<double>(pf) + ql * scale > clo[s][a])
+                            while (ql > 0 && pf + ql * scale > clo[s][a]) ql -= 1.0;
+                            while (pf + qh * scale < chi[s][a]) qh += 1.0;
+                            if (qh > 255.0 || pf + ql * scale > clo[s][a])
                             {
                                 ok = false;
                                 break;
                             }
-                            qlo[a][s] = static_cast<uint8_t>(ql);
-                            qhi[a][s] = static_cast<uint8_t>(qh);
+                            // (boxes of triangles without a number in their coordinates are inverted)
+                            qlo[a][s] = static_cast<uint8_t>(std::min(ql, 255.0));
+                            qhi[a][s] = static_cast<uint8_t>(std::max(qh, 0.0));
                         }
                         if (ok) break;
-                        e++;
-                        if (e > 127) throw std::runtime_error("BVH quantisation exponent overflow");
                     }
-                    expo[a] = e;
+                    if (!fits)
+                    {
+                        // a coarser origin for all axes
+                        unit++;
+                        if (unit > 127) throw std::runtime_error("BVH quantisation exponent overflow");
+                        a = 0;
+                        continue;
+                    }
+                    origin[a] = static_cast<int32_t>(q0);
+                    expo[a] = e - (unit - kScaleBelow8);
+                    a++;
                 }
-                Node8 node{};
-                uint32_t header = static_cast<uint32_t>(expo[0] + 127) | (static_cast<uint32_t>(expo[1] + 127) << 8) |
-                                  (static_cast<uint32_t>(expo[2] + 127) << 16) | (static_cast<uint32_t>(innerMask) << 24);
-                uint32_t pb[3];
-                std::memcpy(pb, p, sizeof(pb));
-                node.w[0] = make_uint4(pb[0], pb[1], pb[2], header);
+                Record8& node = out[record];
+                const uint32_t ez = static_cast<uint32_t>(expo[2]);
+                node.w[0] = make_uint4((static_cast<uint32_t>(origin[0]) << 8) | innerMask,
+                                       (static_cast<uint32_t>(origin[1]) << 8) | static_cast<uint32_t>(unit + kUnitBias8),
+                                       (static_cast<uint32_t>(origin[2]) << 8) | ((ez & 7u) << 5) | static_cast<uint32_t>(expo[0]),
+                                       (block << 8) | ((ez >> 3) << 5) | static_cast<uint32_t>(expo[1]));
                 auto pack8 = [](const uint8_t* q, uint32_t& lo, uint32_t& hi)
                 {
                     lo = static_cast<uint32_t>(q[0]) | (static_cast<uint32_t>(q[1]) << 8) | (static_cast<uint32_t>(q[2]) << 16) | (static_cast<uint32_t>(q[3]) << 24);
@@ -672,12 +734,7 @@ namespace pt
                 pack8(qhi[1], a0, a1);
                 pack8(qhi[2], b0, b1);
                 node.w[3] = make_uint4(a0, a1, b0, b1);
-                node.w[4] = make_uint4(childRef[0], childRef[1], childRef[2], childRef[3]);
-                node.w[5] = make_uint4(childRef[4], childRef[5], childRef[6], childRef[7]);
-                pack8(counts, a0, a1);
-                node.w[6] = make_uint4(a0, a1, leafMask, 0);
-                node.w[7] = make_uint4(0, 0, 0, 0);
-                out[me] = node;
+                masks[block] = block_mask(innerMask, leafMask);
             }
         };
 
@@ -688,6 +745,7 @@ namespace pt
         struct BinaryFlattener
         {
             const BinaryBuilder& bin;
+            const std::vector<uint32_t>& leafRecord;
             std::vector<Node2> out;
             uint32_t maxDepth = 0;
 
@@ -737,7 +795,7 @@ namespace pt
                     if (c.leaf())
                     {
                         if (c.count > 255) throw std::runtime_error("BVH leaf larger than 255 triangles");
-                        ref[i] = c.first;
+                        ref[i] = leafRecord[c.first];
                         count[i] = c.count;
                         leafMask |= 1u << i;
                     }
@@ -796,36 +854,23 @@ namespace pt
         plan.split.assign(binaryNodes, 1);
         plan.wide.assign(binaryNodes, 0);
         plan.plan(root);
-        WideBuilder w{b, plan, {}};
-        w.out.resize(plan.count_wide(root));
-        w.emit(root, 0, 0);
+        WideBuilder w{b, plan, models, {}, {}, {}};
+        const uint32_t wideNodes = plan.count_wide(root);
+        w.prepare(wideNodes, static_cast<uint32_t>(binaryNodes));
+        w.emit(root, 0, 0, 0);
         Bvh8 result;
-        result.nodes = std::move(w.out);
+        result.nodeCount = wideNodes;
         result.depth = w.maxDepth.load();
         if (withBinary)
         {
-            BinaryFlattener f{b, {}, 0};
+            BinaryFlattener f{b, w.leafRecord, {}, 0};
             f.out.reserve(b.nodeCount.load() / 2 + 1);
             f.emit(root, 0);
             result.nodes2 = std::move(f.out);
             result.depth2 = f.maxDepth;
         }
-        result.order = b.idx;
-        result.tris.assign(static_cast<size_t>(n) * kTriangleVec4, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-        for (uint32_t j = 0; j < n; j++)
-        {
-            const uint32_t t = b.idx[j];
-            const float* p0 = positions + (static_cast<size_t>(t) * 3 + 0) * 3;
-            const float* p1 = positions + (static_cast<size_t>(t) * 3 + 1) * 3;
-            const float* p2 = positions + (static_cast<size_t>(t) * 3 + 2) * 3;
-            uint32_t ob = t, mb = models[t];
-            float of, mf;
-            std::memcpy(&of, &ob, 4);
-            std::memcpy(&mf, &mb, 4);
-            result.tris[static_cast<size_t>(j) * kTriangleVec4 + 0] = make_float4(p0[0], p0[1], p0[2], of);
-            result.tris[static_cast<size_t>(j) * kTriangleVec4 + 1] = make_float4(p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2], mf);
-            result.tris[static_cast<size_t>(j) * kTriangleVec4 + 2] = make_float4(p2[0] - p0[0], p2[1] - p0[1], p2[2] - p0[2], 0.0f);
-        }
+        result.records = std::move(w.out);
+        result.masks = std::move(w.masks);
         return result;
     }
 }
@@ -843,60 +888,79 @@ namespace pt
             uint64_t leafTriangles = 0;
         };
 
-        // Exact bounds of a subtree; checks each quantised child box against its subtree.
-        void check_node(CheckState& cs, uint32_t node, double lo[3], double hi[3])
+        // The triangles of a leaf, from its first record: counted, and their exact bounds.
+        void check_leaf(CheckState& cs, uint32_t record, double lo[3], double hi[3])
         {
-            const Node8& n = cs.b.nodes[node];
-            float p[3];
-            std::memcpy(p, &n.w[0], 12);
-            const uint32_t header = n.w[0].w;
-            const uint32_t innerMask = header >> 24;
-            const uint32_t leafMask = n.w[6].z & 0xFFu;
-            const uint32_t* child = reinterpret_cast<const uint32_t*>(&n.w[4]);
-            const uint8_t* counts = reinterpret_cast<const uint8_t*>(&n.w[6]);
+            for (int k = 0; k < 3; k++)
+            {
+                lo[k] = DBL_MAX;
+                hi[k] = -DBL_MAX;
+            }
+            for (int j = 0; j < 255; j++)
+            {
+                const uint32_t t = record < cs.b.records.size() ? cs.b.records[record].w[0].w : kInvalid;
+                if (t >= cs.seen.size())
+                {
+                    cs.violations++;
+                    return;
+                }
+                cs.seen[t]++;
+                cs.leafTriangles++;
+                for (int v = 0; v < 3; v++)
+                    for (int k = 0; k < 3; k++)
+                    {
+                        const double c = cs.positions[(static_cast<size_t>(t) * 3 + v) * 3 + k];
+                        lo[k] = std::min(lo[k], c);
+                        hi[k] = std::max(hi[k], c);
+                    }
+                record = cs.b.records[record].w[2].w;
+                if (record == 0) return;
+            }
+            cs.violations++;  // a chain that does not end
+        }
+
+        // Exact bounds of a subtree; checks each quantised child box against its subtree.
+        void check_node(CheckState& cs, uint32_t record, uint32_t depth, double lo[3], double hi[3])
+        {
+            const Record8& n = cs.b.records[record];
+            const uint32_t h[4] = {n.w[0].x, n.w[0].y, n.w[0].z, n.w[0].w};
+            const uint32_t innerMask = h[0] & 0xFFu;
+            const uint32_t block = h[3] >> 8;
             const uint8_t* q = reinterpret_cast<const uint8_t*>(&n.w[1]);  // qlo x,y,z then qhi x,y,z, 8 each
             for (int k = 0; k < 3; k++)
             {
                 lo[k] = DBL_MAX;
                 hi[k] = -DBL_MAX;
             }
-            for (int s = 0; s < 8; s++)
+            if (block >= cs.b.masks.size() || (cs.b.masks[block] & 0xFFu) != innerMask || depth >= cs.b.depth)
+            {
+                cs.violations++;
+                return;
+            }
+            const uint32_t leafMask = cs.b.masks[block] >> 8;
+            for (uint32_t s = 0; s < kBlockRecords; s++)
             {
                 const bool isInner = (innerMask >> s) & 1u, isLeaf = (leafMask >> s) & 1u;
-                if (!isInner && !isLeaf) continue;
-                double clo[3], chi[3];
-                if (isInner)
-                    check_node(cs, child[s], clo, chi);
-                else
+                const uint32_t child = block * kBlockRecords + s;
+                if (!isInner && !isLeaf)
                 {
-                    for (int k = 0; k < 3; k++)
-                    {
-                        clo[k] = DBL_MAX;
-                        chi[k] = -DBL_MAX;
-                    }
-                    if ((child[s] >> 24) != counts[s]) cs.violations++;
-                    for (uint32_t j = 0; j < counts[s]; j++)
-                    {
-                        const uint32_t t = cs.b.order[(child[s] & 0xFFFFFFu) + j];
-                        cs.seen[t]++;
-                        cs.leafTriangles++;
-                        for (int v = 0; v < 3; v++)
-                            for (int k = 0; k < 3; k++)
-                            {
-                                const double c = cs.positions[(static_cast<size_t>(t) * 3 + v) * 3 + k];
-                                clo[k] = std::min(clo[k], c);
-                                chi[k] = std::max(chi[k], c);
-                            }
-                    }
+                    // an empty slot is a record of zeros
+                    static const Record8 zero{};
+                    if (std::memcmp(&cs.b.records[child], &zero, sizeof(zero)) != 0) cs.violations++;
+                    continue;
                 }
+                double clo[3], chi[3];
+                if (isInner) check_node(cs, child, depth + 1, clo, chi);
+                else check_leaf(cs, child, clo, chi);
                 for (int k = 0; k < 3; k++)
                 {
-                    const int e = static_cast<int>((header >> (8 * k)) & 0xFFu) - 127;
-                    const double scale = std::ldexp(1.0, e);
+                    const int e[3] = {static_cast<int>(h[2] & 31u), static_cast<int>(h[3] & 31u),
+                                      static_cast<int>(((h[2] >> 5) & 7u) | (((h[3] >> 5) & 3u) << 3))};
+                    const int unit = static_cast<int>(h[1] & 0xFFu) - kUnitBias8;
+                    const double scale = std::ldexp(1.0, unit - kScaleBelow8 + e[k]);
+                    const double p = std::ldexp(static_cast<double>(static_cast<int32_t>(h[k]) >> 8), unit);
                     const double qlo = q[k * 8 + s], qhi = q[24 + k * 8 + s];
-                    const double blo = static_cast<double>(p[k]) + qlo * scale;
-                    const double bhi = static_cast<double>(p[k]) + qhi * scale;
-                    if (!(blo <= clo[k] && bhi >= chi[k])) cs.violations++;
+                    if (!(p + qlo * scale <= clo[k] && p + qhi * scale >= chi[k])) cs.violations++;
                     lo[k] = std::min(lo[k], clo[k]);
                     hi[k] = std::max(hi[k], chi[k]);
                 }
@@ -922,25 +986,9 @@ namespace pt
                 double clo[3], chi[3];
                 if ((meta >> (16 + c)) & 1u)
                 {
-                    for (int k = 0; k < 3; k++)
-                    {
-                        clo[k] = DBL_MAX;
-                        chi[k] = -DBL_MAX;
-                    }
-                    const uint32_t count = (meta >> (8 * c)) & 0xFFu;
-                    for (uint32_t j = 0; j < count; j++)
-                    {
-                        const uint32_t t = cs.b.order[ref[c] + j];
-                        cs.seen[t]++;
-                        cs.leafTriangles++;
-                        for (int v = 0; v < 3; v++)
-                            for (int k = 0; k < 3; k++)
-                            {
-                                const double x = cs.positions[(static_cast<size_t>(t) * 3 + v) * 3 + k];
-                                clo[k] = std::min(clo[k], x);
-                                chi[k] = std::max(chi[k], x);
-                            }
-                    }
+                    const uint64_t before = cs.leafTriangles;
+                    check_leaf(cs, ref[c], clo, chi);
+                    if (cs.leafTriangles - before != ((meta >> (8 * c)) & 0xFFu)) cs.violations++;
                 }
                 else
                     check_binary(cs, ref[c], clo, chi);
@@ -958,7 +1006,7 @@ namespace pt
     {
         CheckState cs{b, positions, std::vector<uint32_t>(n, 0)};
         double lo[3], hi[3];
-        check_node(cs, 0, lo, hi);
+        check_node(cs, 0, 0, lo, hi);
         Bvh8Check r;
         r.containmentViolations = cs.violations;
         r.leafTriangles = cs.leafTriangles;

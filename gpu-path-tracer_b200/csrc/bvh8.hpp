@@ -9,11 +9,11 @@ namespace pt
 {
     struct Bvh8
     {
-        std::vector<Node8> nodes;
-        std::vector<float4> tris;      // kTriangleVec4 per triangle, leaf order: (v0, orig), (e1, model), (e2, 0), 0
-        std::vector<uint32_t> order;   // leaf position -> input triangle index
+        std::vector<Record8> records;  // kBlockRecords per block
+        std::vector<uint32_t> masks;   // per block: block_mask of what its slots hold
+        uint32_t nodeCount = 0;        // wide nodes
         uint32_t depth = 0;            // levels of the wide tree
-        std::vector<Node2> nodes2;     // the binary tree the BVH8 is collapsed from, FP32 boxes (same leaf order)
+        std::vector<Node2> nodes2;     // the binary tree the BVH8 is collapsed from, FP32 boxes (leaves in the same records)
         uint32_t depth2 = 0;           // levels of the binary tree
     };
 

@@ -16,7 +16,8 @@
 // 5. Wide nodes level by level from the root: each collects its children from the cost table,
 //    assigns them to slots by octant, quantises their boxes in double precision with outward
 //    rounding and reserves consecutive indices for its inner children with one atomic.
-// 6. Triangle records in Morton order (leaf position k holds the k-th triangle of the sort).
+// 6. Headers and triangle records move into their places in the child blocks, which step 5 assigned
+//    (node j's children are block j + 1).
 //
 // Hits do not depend on the tree (the traversal is conservative and ties go to the smaller input
 // index), so frames equal those of a host-built BVH bit for bit; only the traversal work differs.
@@ -335,16 +336,19 @@ namespace pt
             return static_cast<uint32_t>(q[0]) | (static_cast<uint32_t>(q[1]) << 8) | (static_cast<uint32_t>(q[2]) << 16) | (static_cast<uint32_t>(q[3]) << 24);
         }
 
-        // One level of wide nodes: node `levelBase + w` is binary node level[w]. Inner children get
-        // consecutive indices from *counter and enter nextLevel at (index - nextBase).
-        // capacity: entries of `out` and of nextLevel (an index beyond it is refused and reported).
-        __global__ void emit_level_kernel(const uint32_t* level, uint32_t count, uint32_t levelBase, uint32_t nextBase, uint32_t n,
+        // One level of wide nodes: node `levelBase + w` is binary node level[w].x, its header belongs into
+        // record level[w].y. Inner children get consecutive indices from *counter and enter nextLevel at
+        // (index - nextBase); leaf child k (leaf position) gets its record in leafRecord[k]. Headers go to
+        // headers[node], the header's record to headerRecord[node], the children's kinds to masks[node].
+        // capacity: entries of these arrays and of nextLevel (an index beyond it is refused and reported).
+        __global__ void emit_level_kernel(const uint2* level, uint32_t count, uint32_t levelBase, uint32_t nextBase, uint32_t n,
                                           const float4* lo, const float4* hi, const uint2* child, const uint8_t* how, const uint8_t* split,
-                                          uint32_t* counter, uint32_t* nextLevel, Node8* out, uint32_t capacity, uint32_t* errorFlags)
+                                          uint32_t* counter, uint2* nextLevel, Record8* headers, uint32_t* headerRecord, uint32_t* masks,
+                                          uint32_t* leafRecord, uint32_t capacity, uint32_t* errorFlags)
         {
             for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < count; w += gridDim.x * blockDim.x)
             {
-                const uint32_t b = level[w];
+                const uint32_t b = level[w].x;
                 uint32_t kids[8];
                 bool kidLeaf[8];
                 int nk = 0;
@@ -447,24 +451,22 @@ namespace pt
                 int inner = 0;
                 for (int i = 0; i < nk; i++) inner += kidLeaf[i] ? 0 : 1;
                 const uint32_t firstInner = inner ? atomicAdd(counter, static_cast<uint32_t>(inner)) : 0u;
-                uint32_t childRef[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                uint8_t counts[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                const uint32_t block = levelBase + w + 1u;
                 uint32_t innerMask = 0, leafMask = 0;
                 int r = 0;
                 for (int i = 0; i < nk; i++)
                 {
                     const int s = slotOf[i];
+                    const uint32_t record = block * kBlockRecords + static_cast<uint32_t>(s);
                     if (kidLeaf[i])
                     {
-                        childRef[s] = kids[i] | (1u << 24);  // leaf position (24 bits), one triangle
-                        counts[s] = 1;
+                        leafRecord[kids[i]] = record;
                         leafMask |= 1u << s;
                     }
                     else
                     {
                         const uint32_t at = firstInner + static_cast<uint32_t>(r++);
-                        childRef[s] = at;
-                        if (at < capacity && at >= nextBase) nextLevel[at - nextBase] = kids[i];
+                        if (at < capacity && at >= nextBase) nextLevel[at - nextBase] = make_uint2(kids[i], record);
                         else atomicOr(errorFlags, kBuildErrCapacity);
                         innerMask |= 1u << s;
                     }
@@ -474,8 +476,8 @@ namespace pt
                     atomicOr(errorFlags, kBuildErrCapacity);
                     continue;
                 }
-                // quantisation (WideBuilder::emit): origin rounded down to float, power-of-two scales, every
-                // quantised box checked in double to contain its padded child box
+                // quantisation (WideBuilder::emit): power-of-two scales, origin rounded down to a 24-bit multiple
+                // of a power of two, every quantised box checked in double to contain its padded child box
                 double clo[8][3], chi[8][3];
                 bool valid[8] = {};
                 double plo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, phi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
@@ -490,24 +492,39 @@ namespace pt
                         phi[a] = fmax(phi[a], chi[s][a]);
                     }
                 }
-                float p[3];
+                // origins: multiples of 2^unit that have 24 bits; scales within the header's range of the unit
+                int32_t origin[3];
                 int expo[3];
                 uint8_t qlo[3][8], qhi[3][8];
-                bool overflow = false;
+                int unit = kMinUnit8;
                 for (int a = 0; a < 3; a++)
                 {
-                    float pf = __double2float_rd(plo[a]);
-                    p[a] = pf;
-                    const double ext = phi[a] - static_cast<double>(pf);
-                    int e = -126;
+                    int fe;
+                    frexp(fmax(fabs(plo[a]), 1e-300), &fe);
+                    unit = max(unit, fe - 23);
+                }
+                bool overflow = false;
+                for (int a = 0; a < 3;)
+                {
+                    const double grid = ldexp(1.0, unit);
+                    const double q0 = floor(plo[a] / grid);
+                    const double pf = q0 * grid;
+                    const double ext = phi[a] - pf;
+                    int e = unit - kScaleBelow8;
                     if (ext > 0.0)
                     {
                         int fe;
-                        frexp(ext / 255.0, &fe);
-                        e = max(-126, min(127, fe));
+                        frexp(ext / 255.0, &fe);  // ext/255 = m * 2^fe, m in [0.5, 1)
+                        e = max(e, min(127, fe));
                     }
-                    for (;;)
+                    bool fits = fabs(q0) <= static_cast<double>(kMaxOrigin8);
+                    for (; fits; e++)
                     {
+                        if (e > unit + kScaleAbove8 || e > 127)
+                        {
+                            fits = false;
+                            break;
+                        }
                         const double scale = ldexp(1.0, e);
                         bool ok = true;
                         for (int s = 0; s < 8 && ok; s++)
@@ -521,58 +538,80 @@ namespace pt
                             double ql = floor((clo[s][a] - pf) / scale);
                             double qh = ceil((chi[s][a] - pf) / scale);
                             ql = fmax(0.0, ql);
-                            while (ql > 0 && static_cast<double>(pf) + ql * scale > clo[s][a]) ql -= 1.0;
-                            while (static_cast<double>(pf) + qh * scale < chi[s][a]) qh += 1.0;
-                            if (qh > 255.0 || static_cast<double>(pf) + ql * scale > clo[s][a])
+                            while (ql > 0 && pf + ql * scale > clo[s][a]) ql -= 1.0;
+                            while (pf + qh * scale < chi[s][a]) qh += 1.0;
+                            if (qh > 255.0 || pf + ql * scale > clo[s][a])
                             {
                                 ok = false;
                                 break;
                             }
-                            qlo[a][s] = static_cast<uint8_t>(ql);
-                            qhi[a][s] = static_cast<uint8_t>(qh);
+                            // (boxes of triangles without a number in their coordinates are inverted)
+                            qlo[a][s] = static_cast<uint8_t>(fmin(ql, 255.0));
+                            qhi[a][s] = static_cast<uint8_t>(fmax(qh, 0.0));
                         }
                         if (ok) break;
-                        e++;
-                        if (e > 127)
+                    }
+                    if (!fits)
+                    {
+                        // a coarser origin for all axes
+                        unit++;
+                        if (unit > 127)
                         {
                             overflow = true;
                             break;
                         }
+                        a = 0;
+                        continue;
                     }
-                    if (overflow) break;
-                    expo[a] = e;
+                    origin[a] = static_cast<int32_t>(q0);
+                    expo[a] = e - (unit - kScaleBelow8);
+                    a++;
                 }
                 if (overflow)
                 {
                     atomicOr(errorFlags, kBuildErrExponent);
                     continue;
                 }
-                Node8 node;
-                const uint32_t header = static_cast<uint32_t>(expo[0] + 127) | (static_cast<uint32_t>(expo[1] + 127) << 8) |
-                                        (static_cast<uint32_t>(expo[2] + 127) << 16) | (innerMask << 24);
-                node.w[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), header);
+                Record8 node;
+                const uint32_t ez = static_cast<uint32_t>(expo[2]);
+                node.w[0] = make_uint4((static_cast<uint32_t>(origin[0]) << 8) | innerMask,
+                                       (static_cast<uint32_t>(origin[1]) << 8) | static_cast<uint32_t>(unit + kUnitBias8),
+                                       (static_cast<uint32_t>(origin[2]) << 8) | ((ez & 7u) << 5) | static_cast<uint32_t>(expo[0]),
+                                       (block << 8) | ((ez >> 3) << 5) | static_cast<uint32_t>(expo[1]));
                 node.w[1] = make_uint4(pack4(qlo[0]), pack4(qlo[0] + 4), pack4(qlo[1]), pack4(qlo[1] + 4));
                 node.w[2] = make_uint4(pack4(qlo[2]), pack4(qlo[2] + 4), pack4(qhi[0]), pack4(qhi[0] + 4));
                 node.w[3] = make_uint4(pack4(qhi[1]), pack4(qhi[1] + 4), pack4(qhi[2]), pack4(qhi[2] + 4));
-                node.w[4] = make_uint4(childRef[0], childRef[1], childRef[2], childRef[3]);
-                node.w[5] = make_uint4(childRef[4], childRef[5], childRef[6], childRef[7]);
-                node.w[6] = make_uint4(pack4(counts), pack4(counts + 4), leafMask, 0);
-                node.w[7] = make_uint4(0, 0, 0, 0);
-                out[levelBase + w] = node;
+                headers[levelBase + w] = node;
+                headerRecord[levelBase + w] = level[w].y;
+                masks[levelBase + w] = block_mask(innerMask, leafMask);
             }
         }
 
-        // Triangle records in leaf order (bvh8.cpp, BuildBvh8): (v0, input index), (e1, model), (e2, 0), 0.
-        __global__ void triangle_records_kernel(const float* pos, const uint32_t* models, const uint32_t* sorted, uint32_t n, float4* tris)
+        // Triangle records (bvh8.cpp, WideBuilder::emit_leaf): (v0, input index), (e1, model), (e2, 0), 0;
+        // leaf k is the k-th triangle of the sort.
+        __global__ void triangle_records_kernel(const float* pos, const uint32_t* models, const uint32_t* sorted, const uint32_t* leafRecord,
+                                                uint32_t n, Record8* records)
         {
             for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
             {
                 const uint32_t t = sorted[k];
                 const float* p = pos + static_cast<size_t>(t) * 9;
-                tris[static_cast<size_t>(k) * kTriangleVec4 + 0] = make_float4(p[0], p[1], p[2], __uint_as_float(t));
-                tris[static_cast<size_t>(k) * kTriangleVec4 + 1] = make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], __uint_as_float(models[t]));
-                tris[static_cast<size_t>(k) * kTriangleVec4 + 2] = make_float4(p[6] - p[0], p[7] - p[1], p[8] - p[2], 0.0f);
-                tris[static_cast<size_t>(k) * kTriangleVec4 + 3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float4* w = reinterpret_cast<float4*>(records[leafRecord[k]].w);
+                w[0] = make_float4(p[0], p[1], p[2], __uint_as_float(t));
+                w[1] = make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], __uint_as_float(models[t]));
+                w[2] = make_float4(p[6] - p[0], p[7] - p[1], p[8] - p[2], 0.0f);
+            }
+        }
+
+        // Headers into their records, and the masks of the blocks (block 0: the root's header).
+        __global__ void header_records_kernel(const Record8* headers, const uint32_t* headerRecord, const uint32_t* nodeMasks, uint32_t nodes,
+                                              Record8* records, uint32_t* blockMasks)
+        {
+            for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nodes; j += gridDim.x * blockDim.x)
+            {
+                records[headerRecord[j]] = headers[j];
+                blockMasks[j + 1u] = nodeMasks[j];
+                if (j == 0) blockMasks[0] = block_mask(1u, 0u);
             }
         }
 
@@ -589,7 +628,7 @@ namespace pt
         if (n > kMaxTriangles) return Status::Err(GPT_ERR_CAPACITY, "BVH build failed: scene has more than 2^24 triangles");
         const uint32_t nodes = 2 * n - 1;
         DeviceBuffer triLo, triHi, cent, partLo, partHi, keys, keysSorted, values, sorted, lo, hi, child, clustersA, clustersB, nn, merge, mergePos, keep,
-            keepPos, cost, how, split, levelA, levelB, counter, errorFlags, temp, wide;
+            keepPos, cost, how, split, levelA, levelB, counter, errorFlags, temp, wide, headerRecord, nodeMasks, leafRecord;
         const uint32_t parts = grid_for(n, 256, 1024);
         PT_TRY(triLo.allocate(size_t(n) * 16));
         PT_TRY(triHi.allocate(size_t(n) * 16));
@@ -613,11 +652,15 @@ namespace pt
         PT_TRY(cost.allocate(size_t(nodes) * 8 * 4));
         PT_TRY(how.allocate(size_t(nodes) * 8));
         PT_TRY(split.allocate(size_t(nodes)));
-        PT_TRY(levelA.allocate(size_t(n) * 4));
-        PT_TRY(levelB.allocate(size_t(n) * 4));
+        PT_TRY(levelA.allocate(size_t(n) * 8));
+        PT_TRY(levelB.allocate(size_t(n) * 8));
         PT_TRY(counter.allocate(16));
         PT_TRY(errorFlags.allocate(16));
-        PT_TRY(wide.allocate(size_t(n) * sizeof(Node8)));  // at most one wide node per binary inner node (one for n = 1)
+        // at most one wide node per binary inner node (one for n = 1)
+        PT_TRY(wide.allocate(size_t(n) * sizeof(Record8)));
+        PT_TRY(headerRecord.allocate(size_t(n) * 4));
+        PT_TRY(nodeMasks.allocate(size_t(n) * 4));
+        PT_TRY(leafRecord.allocate(size_t(n) * 4));
         size_t sortBytes = 0, scanBytes = 0;
         PT_CUDA("cub::DeviceRadixSort::SortPairs", cub::DeviceRadixSort::SortPairs(nullptr, sortBytes, keys.get<uint32_t>(), keysSorted.get<uint32_t>(),
                                                                                  values.get<uint32_t>(), sorted.get<uint32_t>(), static_cast<int>(n), 0, 30, s));
@@ -692,19 +735,21 @@ namespace pt
 
         // 5: wide nodes level by level
         const uint32_t one = 1;
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(levelA.get<uint32_t>(), &root, 4, cudaMemcpyHostToDevice, s));
+        const uint2 rootLevel = make_uint2(root, 0u);  // the root's header: record 0
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(levelA.get<uint2>(), &rootLevel, sizeof(rootLevel), cudaMemcpyHostToDevice, s));
         PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(counter.get<uint32_t>(), &one, 4, cudaMemcpyHostToDevice, s));
         uint32_t levelBase = 0, count = 1, depth = 0, allocated = 1;
-        uint32_t* level = levelA.get<uint32_t>();
-        uint32_t* nextLevel = levelB.get<uint32_t>();
+        uint2* level = levelA.get<uint2>();
+        uint2* nextLevel = levelB.get<uint2>();
         while (count > 0)
         {
             depth++;
             if (depth > kMaxStack) return Status::Err(GPT_ERR_CAPACITY, "BVH8 deeper than the traversal stack");
             emit_level_kernel<<<grid_for(count, 128, 16384), 128, 0, s>>>(level, count, levelBase, levelBase + count, n, lo.get<float4>(), hi.get<float4>(),
                                                                           child.get<uint2>(), how.get<uint8_t>(), split.get<uint8_t>(),
-                                                                          counter.get<uint32_t>(), nextLevel, wide.get<Node8>(), n,
-                                                                          errorFlags.get<uint32_t>());
+                                                                          counter.get<uint32_t>(), nextLevel, wide.get<Record8>(),
+                                                                          headerRecord.get<uint32_t>(), nodeMasks.get<uint32_t>(),
+                                                                          leafRecord.get<uint32_t>(), n, errorFlags.get<uint32_t>());
             PT_CUDA("wide nodes", cudaGetLastError());
             uint32_t levelFlags = 0;
             PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&allocated, counter.get<uint32_t>(), 4, cudaMemcpyDeviceToHost, s));
@@ -721,14 +766,20 @@ namespace pt
         if (flags & kBuildErrExponent) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "BVH build failed: BVH quantisation exponent overflow");
         if (flags & kBuildErrCapacity) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide-node index beyond the node array");
         if (flags) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide node's child list did not fit");
-        if (allocated >= (1u << 24)) return Status::Err(GPT_ERR_CAPACITY, "BVH8 has more than 2^24 nodes");
+        if (allocated >= kMaxBlocks) return Status::Err(GPT_ERR_CAPACITY, "BVH8 has more than 2^24 nodes");
 
-        // 6: triangle records; the wide nodes move into an allocation of their exact size
-        PT_TRY(out.tris.allocate(size_t(n) * kTriangleVec4 * sizeof(float4)));
-        triangle_records_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(positions, models, sorted.get<uint32_t>(), n, out.tris.get<float4>());
+        // 6: the child blocks (empty slots stay zero)
+        out.blockCount = allocated + 1u;
+        const size_t blockBytes = size_t(out.blockCount) * kBlockRecords * sizeof(Record8);
+        PT_TRY(out.blocks.allocate(blockBytes));
+        PT_TRY(out.blockMasks.allocate(size_t(out.blockCount) * 4));
+        PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(out.blocks.get<void>(), 0, blockBytes, s));
+        triangle_records_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(positions, models, sorted.get<uint32_t>(), leafRecord.get<uint32_t>(), n,
+                                                                       out.blocks.get<Record8>());
         PT_CUDA("triangle records", cudaGetLastError());
-        PT_TRY(out.nodes.allocate(size_t(allocated) * sizeof(Node8)));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(out.nodes.get<void>(), wide.get<void>(), size_t(allocated) * sizeof(Node8), cudaMemcpyDeviceToDevice, s));
+        header_records_kernel<<<grid_for(allocated, 256, 8192), 256, 0, s>>>(wide.get<Record8>(), headerRecord.get<uint32_t>(), nodeMasks.get<uint32_t>(),
+                                                                             allocated, out.blocks.get<Record8>(), out.blockMasks.get<uint32_t>());
+        PT_CUDA("header records", cudaGetLastError());
         PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(s));
         out.nodeCount = allocated;
         out.depth = depth;

@@ -10,9 +10,10 @@ namespace pt
 {
     struct DeviceBvh
     {
-        DeviceBuffer nodes;        // Node8 records, root first
-        DeviceBuffer tris;         // kTriangleVec4 float4 per triangle, leaf order
+        DeviceBuffer blocks;       // kBlockRecords records per block, the root's block first
+        DeviceBuffer blockMasks;   // uint32 per block: block_mask of what its slots hold
         uint32_t nodeCount = 0;
+        uint32_t blockCount = 0;
         uint32_t depth = 0;        // levels of the wide tree
         uint32_t binaryNodes = 0;  // nodes of the clustered binary tree
         uint32_t rounds = 0;       // clustering rounds

@@ -93,24 +93,23 @@ namespace pt
             std::map<size_t, size_t> free_;
         };
 
-        // All resident scenes in one set of arrays. Node child references, triangle input indices,
+        // All resident scenes in one set of arrays. Child blocks, triangle input indices,
         // material indices of triangles and lights, and alias entries of every appended scene are
         // rebased to the packed arrays, so traversal and shading index them without per-scene base
         // pointers; a ray only needs its scene's root node (SceneEntry).
         struct ScenePack
         {
-            DeviceBuffer nodes, tris, shading, materials, textures, lights, bins, binsPower, entries;
+            DeviceBuffer blocks, shading, materials, textures, lights, bins, binsPower, entries;
             std::vector<SceneEntry> entry;
             std::vector<std::unique_ptr<TextureObject>> textureObjects;
-            uint32_t nodeCount = 0, triangleCount = 0, materialCount = 0, lightCount = 0, depth = 0;
+            uint32_t nodeCount = 0, blockCount = 0, triangleCount = 0, materialCount = 0, lightCount = 0, depth = 0;
             bool modelPresent[kModelCount] = {};
             bool anyTextures = false;
 
             SceneView view() const
             {
                 SceneView v{};
-                v.nodes = nodes.get<Node8>();
-                v.tris = tris.get<float4>();
+                v.records = blocks.get<Record8>();
                 v.shading = shading.get<float4>();
                 v.materials = materials.get<MaterialDev>();
                 v.textures = anyTextures ? textures.get<MaterialTextures>() : nullptr;
@@ -118,7 +117,6 @@ namespace pt
                 v.bins = bins.get<uint4>();
                 v.binsPower = binsPower.get<uint4>();
                 v.lightCount = lightCount;
-                v.nodeCount = nodeCount;
                 v.triangleCount = triangleCount;
                 v.depth = depth;
                 return v;
@@ -139,19 +137,20 @@ namespace pt
             if (p.entry.size() >= kMaxScenes) return Status::Err(GPT_ERR_CAPACITY, "At most 256 resident scenes");
             if (static_cast<uint64_t>(p.nodeCount) + s.nodeCount >= (1ull << 24))
                 return Status::Err(GPT_ERR_CAPACITY, "Resident scenes exceed 2^24 BVH8 nodes");
+            if (static_cast<uint64_t>(p.blockCount) + s.blockCount > kMaxBlocks)
+                return Status::Err(GPT_ERR_CAPACITY, "Resident scenes exceed 2^24 BVH8 blocks");
             if (static_cast<uint64_t>(p.triangleCount) + s.triangleCount > kMaxTriangles)
                 return Status::Err(GPT_ERR_CAPACITY, "Resident scenes exceed 2^24 triangles");
-            DeviceBuffer nn, nt, ns, nm, nl, nb, nbp, ntex, ne;
-            PT_TRY(Grow(nn, p.nodes, size_t(p.nodeCount) * sizeof(Node8), s.nodes, size_t(s.nodeCount) * sizeof(Node8), st));
-            PT_TRY(Grow(nt, p.tris, size_t(p.triangleCount) * kTriangleVec4 * 16, s.tris, size_t(s.triangleCount) * kTriangleVec4 * 16, st));
+            DeviceBuffer nn, ns, nm, nl, nb, nbp, ntex, ne;
+            constexpr size_t kBlockBytes = kBlockRecords * sizeof(Record8);
+            PT_TRY(Grow(nn, p.blocks, p.blockCount * kBlockBytes, s.blocks, s.blockCount * kBlockBytes, st));
             PT_TRY(Grow(ns, p.shading, size_t(p.triangleCount) * 144, s.shading, size_t(s.triangleCount) * 144, st));
             PT_TRY(Grow(nm, p.materials, size_t(p.materialCount) * sizeof(MaterialDev), s.materials, size_t(s.materialCount) * sizeof(MaterialDev), st));
             PT_TRY(Grow(nl, p.lights, size_t(p.lightCount) * 112, s.lights, size_t(s.lightCount) * 112, st));
             PT_TRY(Grow(nb, p.bins, size_t(p.lightCount) * 16, s.bins, size_t(s.lightCount) * 16, st));
             PT_TRY(Grow(nbp, p.binsPower, size_t(p.lightCount) * 16, s.binsPower, size_t(s.lightCount) * 16, st));
-            PT_CUDA("rebase nodes", launch_rebase_nodes(nn.get<Node8>() + p.nodeCount, s.nodeCount, p.nodeCount, p.triangleCount, st));
-            uint32_t* triWords = reinterpret_cast<uint32_t*>(nt.get<float4>() + size_t(p.triangleCount) * kTriangleVec4);
-            PT_CUDA("rebase triangles", launch_rebase_field(triWords + 3, s.triangleCount, kTriangleVec4 * 4, p.triangleCount, false, st));
+            PT_CUDA("rebase blocks", launch_rebase_blocks(nn.get<Record8>() + size_t(p.blockCount) * kBlockRecords, s.blockMasks.get<uint32_t>(),
+                                                          s.blockCount, p.blockCount, p.triangleCount, st));
             uint32_t* shadeWords = reinterpret_cast<uint32_t*>(ns.get<float4>() + size_t(p.triangleCount) * 9);
             PT_CUDA("rebase shading", launch_rebase_field(shadeWords + 27, s.triangleCount, 36, p.materialCount, false, st));
             uint32_t* lightWords = reinterpret_cast<uint32_t*>(nl.get<float4>() + size_t(p.lightCount) * 7);
@@ -178,12 +177,11 @@ namespace pt
                     PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(ntex.get<char>() + oldBytes, 0, addBytes, st));
             }
             std::vector<SceneEntry> entries = p.entry;
-            entries.push_back(SceneEntry{p.nodeCount, p.lightCount, s.lightCount, p.triangleCount});
+            entries.push_back(SceneEntry{p.blockCount, p.lightCount, s.lightCount, p.triangleCount});
             PT_TRY(ne.allocate(entries.size() * sizeof(SceneEntry)));
             PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(ne.get<void>(), entries.data(), entries.size() * sizeof(SceneEntry), cudaMemcpyHostToDevice, st));
             PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(st));
-            p.nodes.swap(nn);
-            p.tris.swap(nt);
+            p.blocks.swap(nn);
             p.shading.swap(ns);
             p.materials.swap(nm);
             p.lights.swap(nl);
@@ -193,6 +191,7 @@ namespace pt
             p.entries.swap(ne);
             p.entry = std::move(entries);
             p.nodeCount += s.nodeCount;
+            p.blockCount += s.blockCount;
             p.triangleCount += s.triangleCount;
             p.materialCount += s.materialCount;
             p.lightCount += s.lightCount;

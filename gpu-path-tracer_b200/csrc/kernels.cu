@@ -102,35 +102,34 @@ namespace pt
         }
     };
 
-    // Triangles [first, first + count) of a leaf (leaf order). Returns false when an any-hit query
+    // The triangles of a leaf, from its first record. Returns false when an any-hit query
     // found an occluder (traversal over); closest hit keeps the best hit in st.hit.
     // FIXED: the query's tMin is the wavefront's constant kMinT (no register holds it).
     template <bool ANY, bool FIXED>
-    __device__ __forceinline__ bool leaf_tests(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t first, uint32_t count,
+    __device__ __forceinline__ bool leaf_tests(const SceneView& sc, TraversalState& st, ColdSlot cold, const uint4* tp,
                                                bool& occluded, uint32_t& work)
     {
         const float tmin = FIXED ? kMinT : st.ray.tmin;
-        work += count << kTestShift;
         const float3 d = cold.direction();
-        for (uint32_t k = 0; k < count; k++)
+        for (;;)
         {
-            const uint4* tp = reinterpret_cast<const uint4*>(sc.tris) + static_cast<size_t>(first + k) * kTriangleVec4;
+            work += 1u << kTestShift;
             uint4 ua, ub;
             ldg8(tp, ua, ub);
             const float4 a = make_float4(__uint_as_float(ua.x), __uint_as_float(ua.y), __uint_as_float(ua.z), __uint_as_float(ua.w));
             const float4 b = make_float4(__uint_as_float(ub.x), __uint_as_float(ub.y), __uint_as_float(ub.z), __uint_as_float(ub.w));
             const float4 c = ldg4(reinterpret_cast<const float4*>(tp + 2));
             float t, u, v;
-            if (!intersect_triangle(a, b, c, st.ray.o, d, t, u, v)) continue;
+            const bool hit = intersect_triangle(a, b, c, st.ray.o, d, t, u, v);
             if (ANY)
             {
-                if (t >= tmin && t < st.hitT)
+                if (hit && t >= tmin && t < st.hitT)
                 {
                     occluded = true;
                     return false;
                 }
             }
-            else
+            else if (hit)
             {
                 // better_hit with the best triangle read from shared memory: it matters only at a tie
                 if (t >= tmin && t <= st.hitT)
@@ -151,8 +150,10 @@ namespace pt
                     }
                 }
             }
+            const uint32_t next = __float_as_uint(c.w);
+            if (next == 0u) return true;
+            tp = sc.records[next].w;
         }
-        return true;
     }
 
     // Slab test of one FP32 box of a binary node against [tmin, tmax]. Each per-axis distance is one
@@ -211,9 +212,9 @@ namespace pt
                                   __uint_as_float(w2.z), __uint_as_float(w2.w), st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT, tn1);
         const uint32_t leafMask = (w3.z >> 16) & 3u;
         if (h0 && (leafMask & 1u))
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, w3.x, w3.z & 0xFFu, occluded, work)) return false;
+            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.x].w, occluded, work)) return false;
         if (h1 && (leafMask & 2u))
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, w3.y, (w3.z >> 8) & 0xFFu, occluded, work)) return false;
+            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.y].w, occluded, work)) return false;
         const bool in0 = h0 && !(leafMask & 1u), in1 = h1 && !(leafMask & 2u);
         if (in0 && in1)
         {
@@ -239,43 +240,29 @@ namespace pt
     __device__ __forceinline__ bool traverse_step(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t* stack, uint32_t stride,
                                                   int stackCap, bool& occluded, uint32_t* errorFlags, uint32_t& work)
     {
-        // stack entry = node << 8 | child slots still to visit (traversal order); an entry with no
-        // slots is a node to visit itself (the root a ray starts with)
+        // stack entry = child block << 8 | inner slots of it still to visit (traversal order, never none)
         if (st.sp == 0) return false;
         uint32_t* top = stack + static_cast<uint32_t>(st.sp - 1) * stride;
         const uint32_t entry = *top;
-        uint32_t node;
-        uint32_t m = entry & 0xFFu;
-        if (m == 0)
-        {
-            node = entry >> 8;
-            st.sp--;
-        }
-        else
-        {
-            const uint32_t i = static_cast<uint32_t>(__ffs(m) - 1);
-            m &= m - 1u;
-            if (m == 0) st.sp--;
-            else *top = (entry & ~0xFFu) | m;
-            const uint32_t parent = entry >> 8;
-            const uint32_t* childRefs = reinterpret_cast<const uint32_t*>(&sc.nodes[parent].w[4]);
-            node = __ldg(childRefs + (i ^ st.ray.oct));
-        }
-        const uint4* nw = sc.nodes[node].w;
+        const uint32_t m = entry & 0xFFu;
+        const uint32_t rest = entry & (entry - 1u);  // the lowest slot bit cleared
+        if ((m & (m - 1u)) == 0) st.sp--;
+        else *top = rest;
+        const uint32_t slot = static_cast<uint32_t>(__ffs(m) - 1) ^ st.ray.oct;
+        const uint4* nw = sc.records[static_cast<size_t>(entry >> 8) * kBlockRecords + slot].w;
         work += kVisit;
         uint4 w0, w1, w2, w3;
         ldg8(nw, w0, w1);
         ldg8(nw + 2, w2, w3);
         const uint32_t hitSlots = intersect_children(w0, w1, w2, w3, st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT);
-        const uint32_t innerSlots = hitSlots & (w0.w >> 24);
-        uint32_t leafOrder = permute_mask(hitSlots & ~(w0.w >> 24), st.ray.oct);
+        const uint32_t innerSlots = hitSlots & w0.x & 0xFFu;
+        uint32_t leafOrder = permute_mask(hitSlots & ~w0.x, st.ray.oct);
         while (leafOrder)
         {
             const uint32_t i = static_cast<uint32_t>(__ffs(leafOrder) - 1);
             leafOrder &= leafOrder - 1u;
-            const uint32_t slot = i ^ st.ray.oct;
-            const uint32_t ref = __ldg(reinterpret_cast<const uint32_t*>(&nw[4]) + slot);
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, ref & 0xFFFFFFu, ref >> 24, occluded, work)) return false;
+            const uint4* tp = sc.records[static_cast<size_t>(w0.w >> 8) * kBlockRecords + (i ^ st.ray.oct)].w;
+            if (!leaf_tests<ANY, FIXED>(sc, st, cold, tp, occluded, work)) return false;
         }
         if (innerSlots)
         {
@@ -284,7 +271,7 @@ namespace pt
                 atomicOr(errorFlags, static_cast<uint32_t>(kErrStackOverflow));
                 return false;
             }
-            stack[static_cast<uint32_t>(st.sp) * stride] = (node << 8) | permute_mask(innerSlots, st.ray.oct);
+            stack[static_cast<uint32_t>(st.sp) * stride] = (w0.w & ~0xFFu) | permute_mask(innerSlots, st.ray.oct);
             st.sp++;
         }
         return true;
@@ -311,7 +298,7 @@ namespace pt
     {
         SceneView sc;
         Wavefront wf;
-        const SceneEntry* scenes;  // nullptr: one scene rooted at node 0
+        const SceneEntry* scenes;  // nullptr: one scene, its root in block 0
         int stackCap = 0;          // traversal stack entries a ray may use (0 = the kernel's whole stack)
         static constexpr int kPhase = 0;
         static constexpr bool kFixedTmin = true;   // every wavefront ray starts at kMinT
@@ -435,7 +422,7 @@ namespace pt
     // Persistent traversal: each warp keeps 32 rays in flight; when at least `refill` lanes are
     // idle the warp takes that many new rays with one atomic (ballot + popc + shuffle), so lanes
     // that finished early are refilled instead of idling until the slowest ray of the warp ends.
-    // Traversal stack: STACK entries per thread in shared memory, entry = node << 8 | child mask.
+    // Traversal stack: STACK entries per thread in shared memory, entry = child block << 8 | child mask.
     // BINARY: the binary FP32 BVH with a per-thread stack of kMaxStack entries in local memory (the
     // plain format); otherwise the BVH8 with the shared-memory stack.
     // Shared memory: [cold slots: 2 x float4 per thread][BVH8 stack: STACK words per thread].
@@ -504,7 +491,8 @@ namespace pt
                         }
                         else
                         {
-                            stack[0] = work.root(tag) << 8;
+                            // the root's block has one record, in slot 0
+                            stack[0] = (work.root(tag) << 8) | (1u << st.ray.oct);
                             st.sp = 1;
                         }
                         active = true;
@@ -2032,19 +2020,20 @@ namespace pt
         }
     }
 
-    // Child references of BVH8 nodes: inner children by nodeOffset, leaf ranges by triOffset.
-    __global__ void rebase_nodes_kernel(Node8* nodes, uint32_t n, uint32_t nodeOffset, uint32_t triOffset)
+    // A scene's blocks appended to the packed array: child blocks move by blockOffset, triangle indices by
+    // triOffset. One thread per record; masks[b] says what a block's slots hold.
+    __global__ void rebase_blocks_kernel(Record8* records, const uint32_t* masks, uint32_t blocks, uint32_t blockOffset, uint32_t triOffset)
     {
+        const uint32_t n = blocks * kBlockRecords;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         {
-            Node8& nd = nodes[i];
-            const uint32_t inner = nd.w[0].w >> 24;
-            const uint32_t leaf = nd.w[6].z & 0xFFu;
-            uint32_t* refs = reinterpret_cast<uint32_t*>(&nd.w[4]);
-            for (int k = 0; k < 8; k++)
+            const uint32_t mask = masks[i / kBlockRecords] >> (i % kBlockRecords);
+            uint4* w = records[i].w;
+            if (mask & 1u) w[0].w += blockOffset << 8;
+            else if ((mask >> 8) & 1u)
             {
-                if ((inner >> k) & 1u) refs[k] += nodeOffset;
-                else if ((leaf >> k) & 1u) refs[k] += triOffset;
+                w[0].w += triOffset;
+                if (w[2].w != 0u) w[2].w += blockOffset * kBlockRecords;
             }
         }
     }
@@ -2308,11 +2297,13 @@ namespace pt
         return cudaGetLastError();
     }
 
-    cudaError_t launch_rebase_nodes(Node8* nodes, uint32_t n, uint32_t nodeOffset, uint32_t triOffset, cudaStream_t s)
+    cudaError_t launch_rebase_blocks(Record8* records, const uint32_t* masks, uint32_t count, uint32_t blockOffset, uint32_t triOffset,
+                                     cudaStream_t s)
     {
-        if (n == 0) return cudaSuccess;
+        if (count == 0) return cudaSuccess;
+        const uint32_t n = count * kBlockRecords;
         const uint32_t blocks = (n + 255) / 256 < 16384 ? (n + 255) / 256 : 16384;
-        rebase_nodes_kernel<<<blocks, 256, 0, s>>>(nodes, n, nodeOffset, triOffset);
+        rebase_blocks_kernel<<<blocks, 256, 0, s>>>(records, masks, count, blockOffset, triOffset);
         return cudaGetLastError();
     }
 

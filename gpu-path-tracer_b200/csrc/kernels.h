@@ -61,7 +61,8 @@ namespace pt
     cudaError_t launch_engine_init(const Wavefront& wf, const EngineView& ev, uint32_t pool, cudaStream_t stream);
     cudaError_t launch_engine_iteration(const EngineLaunch& launch, cudaStream_t stream);
     cudaError_t launch_rebase_field(uint32_t* base, uint32_t n, uint32_t strideWords, uint32_t offset, bool skipInvalid, cudaStream_t stream);
-    cudaError_t launch_rebase_nodes(Node8* nodes, uint32_t n, uint32_t nodeOffset, uint32_t triOffset, cudaStream_t stream);
+    cudaError_t launch_rebase_blocks(Record8* records, const uint32_t* masks, uint32_t blocks, uint32_t blockOffset, uint32_t triOffset,
+                                     cudaStream_t stream);
     cudaError_t launch_iteration(const IterationLaunch& launch, cudaStream_t stream);
     cudaError_t launch_frame_prologue(const Wavefront& wf, const JobView* job, uint32_t pool, int blocks, cudaStream_t stream);
     cudaError_t launch_resolve(const JobView* job, float4* accumulation, uint32_t* framebuffer, int blocks, cudaStream_t stream);

@@ -1,9 +1,8 @@
 // Internal layouts shared by the host runtime (renderer.cu, bvh8.cpp) and the kernels.
 //
 // HBM layout (all structure-of-arrays, 16-byte vector records, one CUDA allocation each):
-//   BVH8 node        128 B  (Node8 below)           scene-resident
-//   triangle (MT)     64 B  v0|orig, e1|model, e2, 0  leaf order, scene-resident (32-byte aligned:
-//                           v0 and e1 in one 256-bit load, e2 in a 128-bit one)
+//   BVH8 child block 512 B  8 records of 64 B (Record8 below): the node headers and triangles that are
+//                           the children of one wide node, scene-resident
 //   triangle shading 144 B  3 normals, 3 tangents, gN|material, uvs (Triangle.hpp:24-38 layout), input order
 //   light           112 B   v0|index, e1|area, e2, gN, emission, uv0|uvE1, uvE2|material
 //   alias bin         16 B  q, p, alias, value (AliasTableView.hpp:8-14); two tables, area and power weights
@@ -34,8 +33,7 @@ namespace pt
     constexpr uint32_t kSlotMask = (1u << kSlotBits) - 1u;
     constexpr uint32_t kMaxPool = 1u << kSlotBits;
     constexpr uint32_t kMaxScenes = 256;
-    constexpr uint32_t kMaxTriangles = 1u << 24;  // leaf references hold 24-bit triangle positions
-    constexpr uint32_t kTriangleVec4 = 4;         // 16-byte words per traversal triangle record (64 B)
+    constexpr uint32_t kMaxTriangles = 1u << 24;  // triangle index and shading model share a word of a hit
     constexpr uint32_t kMaxJobs = 65536;
     constexpr uint32_t kMaxRing = 256;
 
@@ -56,24 +54,40 @@ namespace pt
         kLightsPower = 1,
     };
 
-    // BVH8 node, 128 bytes = 8 x uint4, loaded as one L1 line.
-    //  w[0] = px, py, pz (float bits), ex | ey<<8 | ez<<16 | innerMask<<24   (biased float exponents of the scales)
-    //  w[1] = qlo.x[0..7] (x,y words), qlo.y[0..7] (z,w words)
-    //  w[2] = qlo.z[0..7], qhi.x[0..7]
-    //  w[3] = qhi.y[0..7], qhi.z[0..7]
-    //  w[4], w[5] = child[0..7]: internal -> node index, leaf -> first triangle (leaf order, bits 0-23)
-    //               | triangle count << 24
-    //  w[6] = count[0..7] (bytes, leaf triangle counts), leafMask, 0   (builder and checker only)
-    //  w[7] = reserved
-    // Empty slots hold inverted boxes (lo 255, hi 0) and child reference 0. A node visit reads w[0..3]
-    // (64 bytes); a leaf or a pop reads one child reference.
+    // BVH8: blocks of 8 records of 64 bytes. Block 0 holds the root's header in slot 0; block j + 1 holds
+    // the children of wide node j in their slots: a node header for an inner child, a triangle for a leaf
+    // child, zeros for an empty slot. A child's address follows from the block and the slot alone, so a
+    // step of the traversal is one dependent load (the header or triangle itself): with child references
+    // in the node (128-B nodes, triangles apart) every pop and every leaf first waited for a 4-byte
+    // reference in another sector of the node.
+    //  Node header:
+    //   w[0] = qx << 8 | inner mask, qy << 8 | u, qz << 8 | ez[2:0] << 5 | ex, block << 8 | ez[4:3] << 5 | ey
+    //          origin = q * 2^(u - 119) per axis (q signed, 24 bits: the float precision of its largest
+    //          coordinate), box scale of an axis = 2^(u - 126 + e), block = the node's child block
+    //   w[1] = qlo.x[0..7] (x,y words), qlo.y[0..7] (z,w words)
+    //   w[2] = qlo.z[0..7], qhi.x[0..7]
+    //   w[3] = qhi.y[0..7], qhi.z[0..7]
+    //  Triangle: v0|input index, e1|shading model, e2|next, 0. next = record of the leaf's next triangle,
+    //   0 for the last one (leaves hold one triangle unless the builder's depth limit stopped it; further
+    //   triangles of a leaf lie in the slots of extra blocks behind the nodes').
+    // Empty slots have inverted boxes (lo 255, hi 0); one that the widened box test lets through is a
+    // triangle with zero edges, which no ray hits.
     // Child slots are assigned by octant, so that visiting slot (i ^ rayOctant) for i = 0..7
     // is an approximate front-to-back order.
-    struct __align__(16) Node8
+    struct __align__(32) Record8
     {
-        uint4 w[8];
+        uint4 w[4];
     };
-    static_assert(sizeof(Node8) == 128, "BVH8 node is 128 bytes");
+    static_assert(sizeof(Record8) == 64, "BVH8 records are 64 bytes");
+    constexpr uint32_t kBlockRecords = 8;
+    constexpr uint32_t kMaxBlocks = 1u << 24;          // block indices have 24 bits in headers and stack entries
+    constexpr int32_t kMaxOrigin8 = (1 << 23) - 1;     // largest |q| of a header's origin
+    // Exponents of a header: origins are multiples of 2^U, scales lie between 2^(U - 7) and 2^(U + 24)
+    // (2 units of the origin are about the smallest padded extent), and u = U + 119 is stored.
+    constexpr int kScaleBelow8 = 7, kScaleAbove8 = 24, kUnitBias8 = 119, kMinUnit8 = -118;
+
+    // What a block's slots hold: inner mask in bits 0-7, leaf mask in bits 8-15 (scene packing and checker).
+    constexpr uint32_t block_mask(uint32_t inner, uint32_t leaf) { return inner | (leaf << 8); }
 
     // Binary BVH node with FP32 child boxes, 64 bytes = 4 x uint4 (the plain format, compared with the
     // quantised BVH8 on the same binned-SAH binary tree the BVH8 is collapsed from).
@@ -81,7 +95,7 @@ namespace pt
     //  w[1] = hi0.y, hi0.z, lo1.x, lo1.y
     //  w[2] = lo1.z, hi1.x, hi1.y, hi1.z
     //  w[3] = ref0, ref1, count0 | count1 << 8 | leafMask << 16 | validMask << 24, 0
-    // ref: internal child -> node index, leaf child -> first triangle (leaf order, shared with BVH8).
+    // ref: internal child -> node index, leaf child -> record of its (first) triangle in the BVH8's blocks.
     struct __align__(16) Node2
     {
         uint4 w[4];
@@ -119,8 +133,7 @@ namespace pt
 
     struct SceneView
     {
-        const Node8* nodes;
-        const float4* tris;       // kTriangleVec4 per triangle, leaf order
+        const Record8* records;   // BVH8 blocks, kBlockRecords records each
         const float4* shading;    // 9 per triangle, input order
         const MaterialDev* materials;
         const MaterialTextures* textures;  // per material, nullptr when the scene has no image textures
@@ -128,14 +141,13 @@ namespace pt
         const uint4* bins;        // alias table, area weights (the reference's light sampler)
         const uint4* binsPower;   // alias table, power weights (area x emission luminance)
         uint32_t lightCount;
-        uint32_t nodeCount;
         uint32_t triangleCount;
         uint32_t depth;           // BVH8 depth (stack entries needed)
         const Node2* nodes2;      // binary FP32 BVH of the same scene (frame renderer only), nullptr if absent
         uint32_t depth2;          // binary BVH depth
     };
 
-    // Per resident scene: where its BVH8 starts in the packed node array and its slice of the
+    // Per resident scene: the first of its BVH8 blocks (the root's) in the packed array and its slice of the
     // packed light list / alias table (alias entries are stored rebased to the packed list).
     struct __align__(16) SceneEntry
     {

@@ -208,9 +208,10 @@ namespace pt
             PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(modelsDev.get<void>(), models.data(), static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream));
             DeviceBvh dev;
             PT_TRY(BuildBvh8Device(pos.get<float>(), modelsDev.get<uint32_t>(), n, stream, dev));
-            scene->nodes.swap(dev.nodes);
-            scene->tris.swap(dev.tris);
+            scene->blocks.swap(dev.blocks);
+            scene->blockMasks.swap(dev.blockMasks);
             scene->nodeCount = dev.nodeCount;
+            scene->blockCount = dev.blockCount;
             scene->depth = dev.depth;
             withBinary = false;
         }
@@ -226,13 +227,14 @@ namespace pt
                 return Status::Err(GPT_ERR_INVALID_ARGUMENT, std::string("BVH build failed: ") + e.what());
             }
             if (bvh.depth > kMaxStack) return Status::Err(GPT_ERR_CAPACITY, "BVH8 deeper than the traversal stack");
-            if (bvh.nodes.size() >= (1u << 24)) return Status::Err(GPT_ERR_CAPACITY, "BVH8 has more than 2^24 nodes");
-            scene->nodeCount = static_cast<uint32_t>(bvh.nodes.size());
+            if (bvh.nodeCount >= kMaxBlocks) return Status::Err(GPT_ERR_CAPACITY, "BVH8 has more than 2^24 nodes");
+            scene->nodeCount = bvh.nodeCount;
+            scene->blockCount = static_cast<uint32_t>(bvh.masks.size());
             scene->depth = bvh.depth;
-            PT_TRY(scene->nodes.allocate(bvh.nodes.size() * sizeof(Node8)));
-            PT_TRY(scene->tris.allocate(bvh.tris.size() * sizeof(float4)));
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->nodes.get<void>(), bvh.nodes.data(), bvh.nodes.size() * sizeof(Node8), cudaMemcpyHostToDevice, stream));
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->tris.get<void>(), bvh.tris.data(), bvh.tris.size() * sizeof(float4), cudaMemcpyHostToDevice, stream));
+            PT_TRY(scene->blocks.allocate(bvh.records.size() * sizeof(Record8)));
+            PT_TRY(scene->blockMasks.allocate(bvh.masks.size() * 4));
+            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->blocks.get<void>(), bvh.records.data(), bvh.records.size() * sizeof(Record8), cudaMemcpyHostToDevice, stream));
+            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->blockMasks.get<void>(), bvh.masks.data(), bvh.masks.size() * 4, cudaMemcpyHostToDevice, stream));
         }
         scene->bvhSeconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - tBvh).count();
         rangeBvh.end();
@@ -1288,19 +1290,14 @@ extern "C"
         if (triangle_count != sc->triangleCount)
             return Report(r, pt::Status::Err(GPT_ERR_INVALID_ARGUMENT, "Triangle count differs from the uploaded scene"));
         pt::Bvh8 b;
-        b.nodes.resize(sc->nodeCount);
-        b.tris.resize(static_cast<size_t>(sc->triangleCount) * pt::kTriangleVec4);
+        b.records.resize(static_cast<size_t>(sc->blockCount) * pt::kBlockRecords);
+        b.masks.resize(sc->blockCount);
+        b.nodeCount = sc->nodeCount;
         b.depth = sc->depth;
         cudaError_t e = cudaSetDevice(r->impl->device_);
-        if (e == cudaSuccess) e = cudaMemcpy(b.nodes.data(), sc->nodes.get<void>(), b.nodes.size() * sizeof(pt::Node8), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(b.tris.data(), sc->tris.get<void>(), b.tris.size() * sizeof(float4), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(b.records.data(), sc->blocks.get<void>(), b.records.size() * sizeof(pt::Record8), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(b.masks.data(), sc->blockMasks.get<void>(), b.masks.size() * 4, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return Report(r, pt::CudaStatus("cudaMemcpy", e));
-        b.order.resize(sc->triangleCount);
-        for (uint32_t k = 0; k < sc->triangleCount; k++)
-        {
-            const float w = b.tris[static_cast<size_t>(k) * pt::kTriangleVec4].w;  // input index of leaf position k
-            std::memcpy(&b.order[k], &w, 4);
-        }
         const pt::Bvh8Check c = pt::CheckBvh8(b, positions, triangle_count);
         if (containment_violations) *containment_violations = c.containmentViolations;
         if (triangles_not_exactly_once) *triangles_not_exactly_once = c.trianglesNotExactlyOnce;
@@ -1360,7 +1357,7 @@ extern "C"
             pt::Bvh8 b = pt::BuildBvh8(d->positions, models.data(), d->triangle_count,
                                        static_cast<int>(std::max(1u, std::thread::hardware_concurrency())), true);
             pt::Bvh8Check c = pt::CheckBvh8(b, d->positions, d->triangle_count);
-            if (node_count) *node_count = static_cast<uint32_t>(b.nodes.size());
+            if (node_count) *node_count = b.nodeCount;
             if (depth) *depth = b.depth;
             if (violations) *violations = c.containmentViolations;
             if (misplaced) *misplaced = c.trianglesNotExactlyOnce;

@@ -125,9 +125,9 @@ namespace pt
 
     struct SceneGpu
     {
-        DeviceBuffer nodes, tris, shading, materials, lights, bins, binsPower, materialTextures, entry, nodes2;
+        DeviceBuffer blocks, blockMasks, shading, materials, lights, bins, binsPower, materialTextures, entry, nodes2;
         std::vector<std::unique_ptr<TextureObject>> textures;
-        uint32_t nodeCount = 0, triangleCount = 0, depth = 0, lightCount = 0, materialCount = 0;
+        uint32_t nodeCount = 0, blockCount = 0, triangleCount = 0, depth = 0, lightCount = 0, materialCount = 0;
         uint32_t nodeCount2 = 0, depth2 = 0;  // binary FP32 BVH, built when the scene is uploaded with it
         bool modelPresent[kModelCount] = {};
         uint64_t version = 0;
@@ -136,8 +136,7 @@ namespace pt
         SceneView view() const
         {
             SceneView v{};
-            v.nodes = nodes.get<Node8>();
-            v.tris = tris.get<float4>();
+            v.records = blocks.get<Record8>();
             v.shading = shading.get<float4>();
             v.materials = materials.get<MaterialDev>();
             v.textures = textures.empty() ? nullptr : materialTextures.get<MaterialTextures>();
@@ -145,7 +144,6 @@ namespace pt
             v.bins = bins.get<uint4>();
             v.binsPower = binsPower.get<uint4>();
             v.lightCount = lightCount;
-            v.nodeCount = nodeCount;
             v.triangleCount = triangleCount;
             v.depth = depth;
             v.nodes2 = nodeCount2 ? nodes2.get<Node2>() : nullptr;

@@ -61,23 +61,28 @@ namespace pt
     // distance is lowered and the exit distance raised by 2^-20 of the node's scale in ray
     // space, so the test is conservative for every child box (a box the exact arithmetic
     // would hit is never culled). Returns the hit mask in slot order. Empty slots hold inverted
-    // boxes and are almost always culled; one that passes has a zero child reference (no work).
+    // boxes and are almost always culled; one that passes is a record of zeros, which no ray hits.
     PT_HD uint32_t intersect_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, float tmin, float tmax)
     {
-        const float px = as_float(w0.x), py = as_float(w0.y), pz = as_float(w0.z);
-        const float sx = as_float((w0.w & 0xFFu) << 23);
-        const float sy = as_float(((w0.w >> 8) & 0xFFu) << 23);
-        const float sz = as_float(((w0.w >> 16) & 0xFFu) << 23);
+        // unit = 2^(u - 127) is 2^-8 of the origin's grid (the low byte of a word is masked, so it holds
+        // 256 q); the shift leaves a bit of q in the sign, which fabsf drops. Scales are unit * 2^(e + 1).
+        // Powers of two: origin and scale are exact, and dx, dy, dz round once.
+        const float unit = fabsf(as_float(w0.y << 23));
+        const float sx = as_float(((w0.z << 23) & 0x0F800000u) | 0x40000000u) * unit;
+        const float sy = as_float(((w0.w << 23) & 0x0F800000u) | 0x40000000u) * unit;
+        const float sz = as_float(((w0.z << 18) & 0x03800000u) | ((w0.w << 21) & 0x0C000000u) | 0x40000000u) * unit;
         const float ax = sx * r.invd.x, ay = sy * r.invd.y, az = sz * r.invd.z;
-        const float dx = px - r.o.x, dy = py - r.o.y, dz = pz - r.o.z;
+        const float dx = fma_hd(static_cast<float>(static_cast<int32_t>(w0.x & ~0xFFu)), unit, -r.o.x);
+        const float dy = fma_hd(static_cast<float>(static_cast<int32_t>(w0.y & ~0xFFu)), unit, -r.o.y);
+        const float dz = fma_hd(static_cast<float>(static_cast<int32_t>(w0.z & ~0xFFu)), unit, -r.o.z);
         const float bx = dx * r.invd.x, by = dy * r.invd.y, bz = dz * r.invd.z;
         const float kEps = 9.5367431640625e-07f;  // 2^-20
-        const float ex = (fabsf(dx) + 256.0f * sx) * fabsf(r.invd.x) * kEps;
-        const float ey = (fabsf(dy) + 256.0f * sy) * fabsf(r.invd.y) * kEps;
-        const float ez = (fabsf(dz) + 256.0f * sz) * fabsf(r.invd.z) * kEps;
-        const float bnx = bx - ex, bfx = bx + ex;
-        const float bny = by - ey, bfy = by + ey;
-        const float bnz = bz - ez, bfz = bz + ez;
+        const float ex = fma_hd(256.0f, fabsf(ax), fabsf(bx));
+        const float ey = fma_hd(256.0f, fabsf(ay), fabsf(by));
+        const float ez = fma_hd(256.0f, fabsf(az), fabsf(bz));
+        const float bnx = fma_hd(-kEps, ex, bx), bfx = fma_hd(kEps, ex, bx);
+        const float bny = fma_hd(-kEps, ey, by), bfy = fma_hd(kEps, ey, by);
+        const float bnz = fma_hd(-kEps, ez, bz), bfz = fma_hd(kEps, ez, bz);
         // qlo.x = w1.xy, qlo.y = w1.zw, qlo.z = w2.xy, qhi.x = w2.zw, qhi.y = w3.xy, qhi.z = w3.zw
         const bool nx = r.invd.x < 0.0f, ny = r.invd.y < 0.0f, nz = r.invd.z < 0.0f;
         const uint32_t nxl = nx ? w2.z : w1.x, nxh = nx ? w2.w : w1.y;

@@ -83,7 +83,7 @@ BVH8_Q8, BVH2_FP32 = 0, 1
 BVH_BUILD_HOST, BVH_BUILD_DEVICE = 0, 1
 WAVEFRONT_B200, WAVEFRONT_QUEUES = 0, 1
 SCHEDULE_SHORTEST_FIRST, SCHEDULE_OLDEST_FIRST, SCHEDULE_DEADLINE, SCHEDULE_TWO_CLASS = 1, 2, 3, 4
-NODE_BYTES = {BVH8_Q8: 64 + 4, BVH2_FP32: 64}  # bytes a node visit reads: BVH8 header + its child reference; the whole binary node
+NODE_BYTES = {BVH8_Q8: 64, BVH2_FP32: 64}  # bytes a node visit reads: the BVH8 header; the whole binary node
 
 
 class gpt_frame_stats(ctypes.Structure):

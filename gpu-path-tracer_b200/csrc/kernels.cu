@@ -234,20 +234,31 @@ namespace pt
         return true;
     }
 
-    // Visit one node or pop the next child group. Returns false when traversal is over.
-    // ANY: stops at the first triangle with tmin <= t < tmax.
-    template <bool ANY, bool FIXED>
-    __device__ __forceinline__ bool traverse_step(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t* stack, uint32_t stride,
-                                                  int stackCap, bool& occluded, uint32_t* errorFlags, uint32_t& work)
+    // Bit i of each byte of the result = bit (i ^ oct) of that byte of m.
+    __device__ __forceinline__ uint32_t permute_masks(uint32_t m, uint32_t oct)
     {
-        // stack entry = child block << 8 | inner slots of it still to visit (traversal order, never none)
-        if (st.sp == 0) return false;
+        if (oct & 1u) m = ((m & 0x5555u) << 1) | ((m >> 1) & 0x5555u);
+        if (oct & 2u) m = ((m & 0x3333u) << 2) | ((m >> 2) & 0x3333u);
+        if (oct & 4u) m = ((m & 0x0F0Fu) << 4) | ((m >> 4) & 0x0F0Fu);
+        return m;
+    }
+
+    // Groups of leaf children a lane may hold besides the current one before it stops visiting nodes.
+    constexpr int kLeafQueue = 2;
+    // Leaves are tested once 1 / kLeafShare of the warp's busy lanes have some waiting.
+    constexpr int kLeafShare = 3;
+
+    // One node visit of the BVH8. leaves: group of leaf children waiting for their tests (block << 8 |
+    // slots in traversal order, 0 = none), waiting: further groups in queue[].
+    template <bool FIXED>
+    __device__ __forceinline__ void visit_node(const SceneView& sc, TraversalState& st, uint32_t* stack, uint32_t stride, int stackCap,
+                                               uint32_t& leaves, int& waiting, uint32_t* queue, uint32_t* errorFlags, uint32_t& work)
+    {
         uint32_t* top = stack + static_cast<uint32_t>(st.sp - 1) * stride;
         const uint32_t entry = *top;
         const uint32_t m = entry & 0xFFu;
-        const uint32_t rest = entry & (entry - 1u);  // the lowest slot bit cleared
         if ((m & (m - 1u)) == 0) st.sp--;
-        else *top = rest;
+        else *top = entry & (entry - 1u);
         const uint32_t slot = static_cast<uint32_t>(__ffs(m) - 1) ^ st.ray.oct;
         const uint4* nw = sc.records[static_cast<size_t>(entry >> 8) * kBlockRecords + slot].w;
         work += kVisit;
@@ -255,26 +266,54 @@ namespace pt
         ldg8(nw, w0, w1);
         ldg8(nw + 2, w2, w3);
         const uint32_t hitSlots = intersect_children(w0, w1, w2, w3, st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT);
-        const uint32_t innerSlots = hitSlots & w0.x & 0xFFu;
-        uint32_t leafOrder = permute_mask(hitSlots & ~w0.x, st.ray.oct);
-        while (leafOrder)
-        {
-            const uint32_t i = static_cast<uint32_t>(__ffs(leafOrder) - 1);
-            leafOrder &= leafOrder - 1u;
-            const uint4* tp = sc.records[static_cast<size_t>(w0.w >> 8) * kBlockRecords + (i ^ st.ray.oct)].w;
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, tp, occluded, work)) return false;
-        }
-        if (innerSlots)
+        const uint32_t inner = hitSlots & w0.x & 0xFFu;
+        const uint32_t both = permute_masks(inner | ((hitSlots & ~w0.x) << 8), st.ray.oct);
+        const uint32_t block = w0.w & ~0xFFu;
+        if (both & 0xFFu)
         {
             if (st.sp >= stackCap)
             {
                 atomicOr(errorFlags, static_cast<uint32_t>(kErrStackOverflow));
-                return false;
+                st.sp = 0;
+                leaves = 0;
+                waiting = 0;
+                return;
             }
-            stack[static_cast<uint32_t>(st.sp) * stride] = (w0.w & ~0xFFu) | permute_mask(innerSlots, st.ray.oct);
+            stack[static_cast<uint32_t>(st.sp) * stride] = block | (both & 0xFFu);
             st.sp++;
         }
-        return true;
+        if (both >> 8)
+        {
+            if (leaves != 0)
+            {
+                queue[static_cast<uint32_t>(waiting) * stride] = leaves;
+                waiting++;
+            }
+            leaves = block | (both >> 8);
+        }
+    }
+
+    // Tests the next triangle of the lane's waiting leaves. An any-hit query that finds an occluder ends.
+    template <bool ANY, bool FIXED>
+    __device__ __forceinline__ void test_leaf(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t& leaves, int& waiting,
+                                              const uint32_t* queue, uint32_t stride, uint32_t& work)
+    {
+        const uint32_t slot = static_cast<uint32_t>(__ffs(leaves & 0xFFu) - 1) ^ st.ray.oct;
+        const uint4* tp = sc.records[static_cast<size_t>(leaves >> 8) * kBlockRecords + slot].w;
+        leaves &= leaves - 1u;
+        if ((leaves & 0xFFu) == 0)
+        {
+            leaves = 0;
+            if (waiting > 0) leaves = queue[static_cast<uint32_t>(--waiting) * stride];
+        }
+        bool occluded = false;
+        if (!leaf_tests<ANY, FIXED>(sc, st, cold, tp, occluded, work))
+        {
+            cold.p[1].z = __uint_as_float(0u);
+            st.sp = 0;
+            leaves = 0;
+            waiting = 0;
+        }
     }
 
     // A path left its slot: counted for the iteration and recorded for regeneration, in the finished-slot
@@ -422,28 +461,15 @@ namespace pt
     // Persistent traversal: each warp keeps 32 rays in flight; when at least `refill` lanes are
     // idle the warp takes that many new rays with one atomic (ballot + popc + shuffle), so lanes
     // that finished early are refilled instead of idling until the slowest ray of the warp ends.
-    // Traversal stack: STACK entries per thread in shared memory, entry = child block << 8 | child mask.
-    // BINARY: the binary FP32 BVH with a per-thread stack of kMaxStack entries in local memory (the
-    // plain format); otherwise the BVH8 with the shared-memory stack.
-    // Shared memory: [cold slots: 2 x float4 per thread][BVH8 stack: STACK words per thread].
-    template <int STACK, bool ANY, int MINB, bool BINARY, class Work>
-    __global__ void __launch_bounds__(128, MINB) trace_kernel(Work work, uint32_t refill, uint32_t* errorFlags)
+    // The plain format: the binary FP32 BVH with a per-thread stack of kMaxStack entries in local memory.
+    // Shared memory: [cold slots: 2 x float4 per thread].
+    template <bool ANY, class Work>
+    __global__ void __launch_bounds__(128, 1) trace_binary_kernel(Work work, uint32_t refill, uint32_t* errorFlags)
     {
         extern __shared__ float4 smem4[];
-        uint32_t localStack[BINARY ? kMaxStack : 1];
-        uint32_t* stack;
-        uint32_t stride;
+        constexpr int STACK = kMaxStack;
+        uint32_t stack[STACK];
         const ColdSlot cold{smem4 + 2u * threadIdx.x};
-        if constexpr (BINARY)
-        {
-            stack = localStack;
-            stride = 1;
-        }
-        else
-        {
-            stack = reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + threadIdx.x;
-            stride = blockDim.x;
-        }
         Counters* ctr = work.counters();
         phase_begin(ctr, Work::kPhase);
         const uint32_t n = work.count();
@@ -484,17 +510,8 @@ namespace pt
                         // of 15.0 node visits per shadow ray). The order changes no result.
                         if (ANY) st.ray.oct ^= 7u;
                         st.hitT = tmax;
-                        if constexpr (BINARY)
-                        {
-                            st.pending = work.root(tag);
-                            st.sp = 0;
-                        }
-                        else
-                        {
-                            // the root's block has one record, in slot 0
-                            stack[0] = (work.root(tag) << 8) | (1u << st.ray.oct);
-                            st.sp = 1;
-                        }
+                        st.pending = work.root(tag);
+                        st.sp = 0;
                         active = true;
                     }
                 }
@@ -511,10 +528,7 @@ namespace pt
 #pragma unroll 1
                 for (int k = 0; k < 4 && more; k++)
                 {
-                    if constexpr (BINARY)
-                        more = traverse_step_binary<ANY, Work::kFixedTmin>(work.sc, st, cold, stack, cap, occluded, errorFlags, counts);
-                    else
-                        more = traverse_step<ANY, Work::kFixedTmin>(work.sc, st, cold, stack, stride, cap, occluded, errorFlags, counts);
+                    more = traverse_step_binary<ANY, Work::kFixedTmin>(work.sc, st, cold, stack, cap, occluded, errorFlags, counts);
                 }
                 if (!more)
                 {
@@ -536,6 +550,131 @@ namespace pt
                     atomicAdd(&ctr->triTests[ANY ? 1 : 0], static_cast<unsigned long long>(counts >> kTestShift));
                     counts = 0;
                 }
+            }
+        }
+        if (ctr != nullptr)
+        {
+            unsigned long long v = counts & 0xFFFFu, t = counts >> kTestShift;
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+                t += __shfl_down_sync(0xFFFFFFFFu, t, o);
+            }
+            if (lane == 0)
+            {
+                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], v);
+                atomicAdd(&ctr->triTests[ANY ? 1 : 0], t);
+            }
+        }
+        phase_end(ctr, Work::kPhase);
+    }
+
+
+    // The same for the BVH8, with the warp's lanes in step: each step visits one node per lane, then tests
+    // one triangle per lane if enough lanes hold leaves (kLeafShare), and goes on testing while more than
+    // half of the busy lanes do. A node visit rarely enters leaves in more than a few lanes (0.34 tests per
+    // visit on spheres-1m), so testing them at once ran the triangle test for 7, then 2, then 1 lane of the
+    // warp and waited for each test's loads; held back, the tests of several visits run together: 16.9
+    // instead of 12.2 active lanes per instruction and 203 M instead of 244 M instructions in a launch of
+    // 2.1 M rays, for 2 % more node visits and 2 % more tests. Frame of spheres-1m (1920x1080x64): 102.7 ->
+    // 92.7 ms; a share of 1/2, 1/4 or 1/8 measured 92.5, 91.8, 92.1 (before the loop), a fixed 6, 16 or 22
+    // lanes 92.2, 97.8, 124 and 1.7 times the time of small batches, whose warps are seldom full. Without
+    // the loop the Cornell box, with its 1.3 tests per visit, took 5.06 instead of 4.77 ms.
+    // Finished rays stay in their lanes until the next refill, which retires them together.
+    // Traversal stack: STACK entries per thread, entry = child block << 8 | child mask.
+    // Shared memory: [cold slots: 2 x float4 per thread][stack: STACK words per thread][kLeafQueue words per thread].
+    template <int STACK, bool ANY, int MINB, class Work>
+    __global__ void __launch_bounds__(128, MINB) trace_kernel(Work work, uint32_t refill, uint32_t* errorFlags)
+    {
+        extern __shared__ float4 smem4[];
+        const ColdSlot cold{smem4 + 2u * threadIdx.x};
+        const uint32_t stride = blockDim.x;
+        uint32_t* stack = reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + threadIdx.x;
+        uint32_t* queue = stack + STACK * stride;
+        Counters* ctr = work.counters();
+        phase_begin(ctr, Work::kPhase);
+        const uint32_t n = work.count();
+        const int cap = (work.stackCap > 0 && work.stackCap < STACK) ? work.stackCap : STACK;
+        uint32_t counts = 0;  // node visits | triangle tests << 16
+        const uint32_t lane = lane_id();
+        TraversalState st;
+        st.sp = 0;
+        uint32_t leaves = 0;
+        int waiting = 0;
+        bool active = false;     // a ray in flight (finished or not)
+        bool exhausted = false;
+        for (;;)
+        {
+            const bool over = st.sp == 0 && leaves == 0;
+            const unsigned idle = __ballot_sync(0xFFFFFFFFu, over);
+            const uint32_t idleCount = static_cast<uint32_t>(__popc(idle));
+            if (idleCount >= refill || idle == 0xFFFFFFFFu)
+            {
+                if (over && active)
+                {
+                    const float4 c0 = cold.p[0], c1 = cold.p[1];
+                    const uint32_t best = __float_as_uint(c1.z);
+                    HitRecord h;
+                    h.t = st.hitT;
+                    h.tri = best == kInvalid ? kInvalid : (best & 0xFFFFFFu);
+                    h.u = c1.x;
+                    h.v = c1.y;
+                    h.model = best == kInvalid ? 0u : (best >> 24);
+                    work.finish(__float_as_uint(c1.w), __float_as_uint(c0.w), h, ANY && best != kInvalid, st.ray.o, make_float3(c0.x, c0.y, c0.z));
+                    active = false;
+                }
+                if (exhausted)
+                {
+                    if (idle == 0xFFFFFFFFu) break;
+                }
+                else
+                {
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(work.cursor(), idleCount);
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                    if (base >= n) exhausted = true;
+                    if (over)
+                    {
+                        unsigned laneMaskLt;
+                        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(laneMaskLt));
+                        const uint32_t i = base + static_cast<uint32_t>(__popc(idle & laneMaskLt));
+                        if (i < n)
+                        {
+                            float3 o, d;
+                            float tmin, tmax;
+                            uint32_t tag;
+                            work.load(i, o, d, tmin, tmax, tag);
+                            cold.p[0] = make_float4(d.x, d.y, d.z, __uint_as_float(tag));
+                            cold.p[1] = make_float4(0.0f, 0.0f, __uint_as_float(kInvalid), __uint_as_float(i));
+                            st.ray = make_ray(o, d, tmin);
+                            if (ANY) st.ray.oct ^= 7u;
+                            st.hitT = tmax;
+                            stack[0] = (work.root(tag) << 8) | (1u << st.ray.oct);
+                            st.sp = 1;
+                            active = true;
+                        }
+                    }
+                    continue;
+                }
+            }
+            if (st.sp > 0 && waiting < kLeafQueue)
+                visit_node<Work::kFixedTmin>(work.sc, st, stack, stride, cap, leaves, waiting, queue, errorFlags, counts);
+            unsigned holding = __ballot_sync(0xFFFFFFFFu, leaves != 0);
+            const unsigned busy = holding | __ballot_sync(0xFFFFFFFFu, st.sp > 0);
+            if (__popc(holding) * kLeafShare >= __popc(busy))
+            {
+                do
+                {
+                    if (leaves != 0) test_leaf<ANY, Work::kFixedTmin>(work.sc, st, cold, leaves, waiting, queue, stride, counts);
+                    holding = __ballot_sync(0xFFFFFFFFu, leaves != 0);
+                } while (__popc(holding) * 2 > __popc(busy));
+            }
+            // a step adds at most one visit and 255 tests: flush the packed counters well before a field overflows
+            if (ctr != nullptr && (counts & 0x80008000u))
+            {
+                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], static_cast<unsigned long long>(counts & 0xFFFFu));
+                atomicAdd(&ctr->triTests[ANY ? 1 : 0], static_cast<unsigned long long>(counts >> kTestShift));
+                counts = 0;
             }
         }
         if (ctr != nullptr)
@@ -2075,8 +2214,8 @@ namespace pt
         template <int STACK, bool ANY, int MINB, class Work>
         cudaError_t launch_trace_t(const Work& w, int blocks, int threads, uint32_t refill, uint32_t* err, cudaStream_t s)
         {
-            const size_t smem = static_cast<size_t>(STACK) * threads * sizeof(uint32_t) + kColdBytes * threads;
-            trace_kernel<STACK, ANY, MINB, false, Work><<<blocks, threads, smem, s>>>(w, refill, err);
+            const size_t smem = static_cast<size_t>(STACK + kLeafQueue) * threads * sizeof(uint32_t) + kColdBytes * threads;
+            trace_kernel<STACK, ANY, MINB, Work><<<blocks, threads, smem, s>>>(w, refill, err);
             return cudaGetLastError();
         }
 
@@ -2084,7 +2223,7 @@ namespace pt
         template <bool ANY, class Work>
         cudaError_t launch_trace_binary(const Work& w, int blocks, int threads, uint32_t refill, uint32_t* err, cudaStream_t s)
         {
-            trace_kernel<kMaxStack, ANY, 1, true, Work><<<blocks, threads, kColdBytes * threads, s>>>(w, refill, err);
+            trace_binary_kernel<ANY, Work><<<blocks, threads, kColdBytes * threads, s>>>(w, refill, err);
             return cudaGetLastError();
         }
 
@@ -2110,8 +2249,8 @@ namespace pt
         int resident_blocks(int threads)
         {
             int perSm = 0;
-            const size_t smem = static_cast<size_t>(STACK) * threads * sizeof(uint32_t) + kColdBytes * threads;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, trace_kernel<STACK, false, MINB, false, WavefrontClosest>, threads, smem);
+            const size_t smem = static_cast<size_t>(STACK + kLeafQueue) * threads * sizeof(uint32_t) + kColdBytes * threads;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, trace_kernel<STACK, false, MINB, WavefrontClosest>, threads, smem);
             return perSm;
         }
 
@@ -2132,7 +2271,7 @@ namespace pt
         if (bvhFormat == kBvh2Fp32)
         {
             perSm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, trace_kernel<kMaxStack, false, 1, true, WavefrontClosest>, threads,
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, trace_binary_kernel<false, WavefrontClosest>, threads,
                                                           kColdBytes * threads);
             return sms * (perSm < 1 ? 1 : perSm);
         }

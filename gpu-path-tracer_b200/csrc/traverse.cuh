@@ -33,15 +33,6 @@ namespace pt
         return r;
     }
 
-    // bit i of the result = bit (i ^ oct) of m: slot order -> traversal order (and back).
-    PT_HD uint32_t permute_mask(uint32_t m, uint32_t oct)
-    {
-        if (oct & 1u) m = ((m & 0x55u) << 1) | ((m & 0xAAu) >> 1);
-        if (oct & 2u) m = ((m & 0x33u) << 2) | ((m & 0xCCu) >> 2);
-        if (oct & 4u) m = ((m & 0x0Fu) << 4) | ((m & 0xF0u) >> 4);
-        return m;
-    }
-
     PT_HD float byte_to_float(uint32_t lo, uint32_t hi, int s)
     {
         const uint32_t w = s < 4 ? lo : hi;

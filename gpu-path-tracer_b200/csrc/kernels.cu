@@ -2210,7 +2210,11 @@ namespace pt
 
         // Traversal kernel variants: stack capacity (>= BVH8 depth) x occupancy target. MINB is the
         // minimum resident 128-thread blocks per SM the compiler must allow (1 = registers unconstrained,
-        // 10 = <= 48 registers, 12 = <= 40 registers); the best one is measured, not assumed.
+        // 9 = <= 56 registers, 12 = <= 40 registers); the best one is measured, not assumed. The default was 10
+        // blocks with 48 registers; with the leaf queue's state these spilled (spheres-1m frame 90.3 ms,
+        // 9 blocks 88.9 ms, 8 blocks with 64 registers 90.9 ms).
+        constexpr int kDefaultBlocks = 9;
+
         template <int STACK, bool ANY, int MINB, class Work>
         cudaError_t launch_trace_t(const Work& w, int blocks, int threads, uint32_t refill, uint32_t* err, cudaStream_t s)
         {
@@ -2231,7 +2235,7 @@ namespace pt
         cudaError_t launch_trace_m(const Work& w, int occupancy, int blocks, int threads, uint32_t refill, uint32_t* err, cudaStream_t s)
         {
             if (occupancy >= 12) return launch_trace_t<STACK, ANY, 12>(w, blocks, threads, refill, err, s);
-            if (occupancy >= 10) return launch_trace_t<STACK, ANY, 10>(w, blocks, threads, refill, err, s);
+            if (occupancy >= 10) return launch_trace_t<STACK, ANY, kDefaultBlocks>(w, blocks, threads, refill, err, s);
             return launch_trace_t<STACK, ANY, 1>(w, blocks, threads, refill, err, s);
         }
 
@@ -2258,7 +2262,7 @@ namespace pt
         int resident_blocks_m(int occupancy, int threads)
         {
             if (occupancy >= 12) return resident_blocks<STACK, 12>(threads);
-            if (occupancy >= 10) return resident_blocks<STACK, 10>(threads);
+            if (occupancy >= 10) return resident_blocks<STACK, kDefaultBlocks>(threads);
             return resident_blocks<STACK, 1>(threads);
         }
     }

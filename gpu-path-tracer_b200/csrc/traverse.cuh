@@ -33,72 +33,121 @@ namespace pt
         return r;
     }
 
-    PT_HD float byte_to_float(uint32_t lo, uint32_t hi, int s)
+    // Node test. Per child it converts 6 bytes, does 6 multiply-adds, 4 min/max and collects one bit. Byte to
+    // float conversions run on the XU pipe (16 a clock per SM), which was the busiest one: 48 of them per visit
+    // kept it 62 % busy with 1.5 warps waiting for it per issue. So one axis gets its bytes by a byte permute
+    // (ALU pipe) as 1 + q / 32768, the bias folded into the axis' offset. Frame of spheres-1m (1920x1080x64): no
+    // axis 92.6 ms, one 90.3, two 91.5, three about 93 (the ALU pipe, which runs the min/max, is then the
+    // busier one). Three-input min/max and the sign of (exit - entry) shifted into the mask take 2 fewer ALU
+    // operations per child than two-input ones and a compare and select (0.9 ms). Packed f32x2 multiply-adds
+    // need their operands in register pairs and were 1 ms slower.
+    template <int K>
+    __device__ __forceinline__ float byte_of(uint32_t w)
     {
-        const uint32_t w = s < 4 ? lo : hi;
-        return static_cast<float>((w >> (8 * (s & 3))) & 0xFFu);
+        return static_cast<float>((w >> (8 * K)) & 0xFFu);
+    }
+    template <int K>
+    __device__ __forceinline__ float biased_byte_of(uint32_t w)  // 1 + q / 32768: the byte in the middle of the mantissa
+    {
+        return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | (static_cast<uint32_t>(K) << 4)));
     }
 
-    PT_HD float fma_hd(float a, float b, float c)
+    // One axis of a node in ray space: plane q lies at q a + b, with b lowered for near planes and raised for
+    // far ones. Rounding of b and of the multiply-add is below 5 ulp of (|b| + 256 |a|), and 2^-20 of it is
+    // taken. A biased axis keeps 32768 a in `a` and b - 32768 a in the offsets, whose rounding is at most
+    // 2^-9 |a|; 2^-8 |a| is taken. Where 32768 a overflows, the planes become NaN, which the min/max ignore.
+    struct SlabAxis
     {
-#ifdef __CUDA_ARCH__
-        return __fmaf_rn(a, b, c);
-#else
-        return fmaf(a, b, c);
-#endif
+        float a, near, far;
+        uint32_t nearLo, nearHi, farLo, farHi;  // bytes of the planes the ray meets first and last, children 0-3 and 4-7
+    };
+
+    template <bool BIASED>
+    __device__ __forceinline__ SlabAxis slab_axis(float origin, float scale, float invd, uint32_t loLo, uint32_t loHi, uint32_t hiLo, uint32_t hiHi)
+    {
+        const float kEps = 9.5367431640625e-07f;  // 2^-20
+        SlabAxis s;
+        s.a = scale * invd;  // (scale: 32768 times the axis' scale when BIASED)
+        const float b = origin * invd;
+        const float e = __fmaf_rn(BIASED ? 0.125f : 256.0f, fabsf(s.a), fabsf(b));
+        s.near = __fmaf_rn(-kEps, e, b);
+        s.far = __fmaf_rn(kEps, e, b);
+        if constexpr (BIASED)
+        {
+            s.near = __fsub_rn(s.near, s.a);
+            s.far = __fsub_rn(s.far, s.a);
+        }
+        const bool negative = invd < 0.0f;
+        s.nearLo = negative ? hiLo : loLo;
+        s.nearHi = negative ? hiHi : loHi;
+        s.farLo = negative ? loLo : hiLo;
+        s.farHi = negative ? loHi : hiHi;
+        return s;
     }
 
-    // Slab test of the 8 quantised children against [tmin, tmax]. The computed entry
-    // distance is lowered and the exit distance raised by 2^-20 of the node's scale in ray
-    // space, so the test is conservative for every child box (a box the exact arithmetic
-    // would hit is never culled). Returns the hit mask in slot order. Empty slots hold inverted
+    template <int S, bool BIASED>
+    __device__ __forceinline__ float slab_plane(uint32_t lo, uint32_t hi, float a, float b)
+    {
+        const uint32_t w = S < 4 ? lo : hi;
+        if constexpr (BIASED) return __fmaf_rn(biased_byte_of<(S & 3)>(w), a, b);
+        else return __fmaf_rn(byte_of<(S & 3)>(w), a, b);
+    }
+
+    __device__ __forceinline__ float max3f(float a, float b, float c)
+    {
+        float r;
+        asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+        return r;
+    }
+    __device__ __forceinline__ float min3f(float a, float b, float c)
+    {
+        float r;
+        asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+        return r;
+    }
+
+    // Shifts 1 into `missed` when the ray misses child S, else 0.
+    template <int S>
+    __device__ __forceinline__ void slab_child(const SlabAxis& x, const SlabAxis& y, const SlabAxis& z, float tmin, float tmax, uint32_t& missed)
+    {
+        const float tn = fmaxf(max3f(slab_plane<S, true>(x.nearLo, x.nearHi, x.a, x.near), slab_plane<S, false>(y.nearLo, y.nearHi, y.a, y.near),
+                                     slab_plane<S, false>(z.nearLo, z.nearHi, z.a, z.near)),
+                               tmin);
+        const float tf = fminf(min3f(slab_plane<S, true>(x.farLo, x.farHi, x.a, x.far), slab_plane<S, false>(y.farLo, y.farHi, y.a, y.far),
+                                     slab_plane<S, false>(z.farLo, z.farHi, z.a, z.far)),
+                               tmax);
+        missed = __funnelshift_l(__float_as_uint(tf - tn), missed, 1);
+    }
+
+    // Slab test of the 8 quantised children against [tmin, tmax], conservative for every child box (a box the
+    // exact arithmetic would hit is never culled). Returns the hit mask in slot order. Empty slots hold inverted
     // boxes and are almost always culled; one that passes is a record of zeros, which no ray hits.
-    PT_HD uint32_t intersect_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, float tmin, float tmax)
+    __device__ __forceinline__ uint32_t intersect_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, float tmin, float tmax)
     {
         // unit = 2^(u - 127) is 2^-8 of the origin's grid (the low byte of a word is masked, so it holds
         // 256 q); the shift leaves a bit of q in the sign, which fabsf drops. Scales are unit * 2^(e + 1).
         // Powers of two: origin and scale are exact, and dx, dy, dz round once.
         const float unit = fabsf(as_float(w0.y << 23));
-        const float sx = as_float(((w0.z << 23) & 0x0F800000u) | 0x40000000u) * unit;
+        const float sx = as_float(((w0.z << 23) & 0x0F800000u) | 0x40000000u) * (unit * 32768.0f);
         const float sy = as_float(((w0.w << 23) & 0x0F800000u) | 0x40000000u) * unit;
         const float sz = as_float(((w0.z << 18) & 0x03800000u) | ((w0.w << 21) & 0x0C000000u) | 0x40000000u) * unit;
-        const float ax = sx * r.invd.x, ay = sy * r.invd.y, az = sz * r.invd.z;
-        const float dx = fma_hd(static_cast<float>(static_cast<int32_t>(w0.x & ~0xFFu)), unit, -r.o.x);
-        const float dy = fma_hd(static_cast<float>(static_cast<int32_t>(w0.y & ~0xFFu)), unit, -r.o.y);
-        const float dz = fma_hd(static_cast<float>(static_cast<int32_t>(w0.z & ~0xFFu)), unit, -r.o.z);
-        const float bx = dx * r.invd.x, by = dy * r.invd.y, bz = dz * r.invd.z;
-        const float kEps = 9.5367431640625e-07f;  // 2^-20
-        const float ex = fma_hd(256.0f, fabsf(ax), fabsf(bx));
-        const float ey = fma_hd(256.0f, fabsf(ay), fabsf(by));
-        const float ez = fma_hd(256.0f, fabsf(az), fabsf(bz));
-        const float bnx = fma_hd(-kEps, ex, bx), bfx = fma_hd(kEps, ex, bx);
-        const float bny = fma_hd(-kEps, ey, by), bfy = fma_hd(kEps, ey, by);
-        const float bnz = fma_hd(-kEps, ez, bz), bfz = fma_hd(kEps, ez, bz);
+        const float dx = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.x & ~0xFFu)), unit, -r.o.x);
+        const float dy = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.y & ~0xFFu)), unit, -r.o.y);
+        const float dz = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.z & ~0xFFu)), unit, -r.o.z);
         // qlo.x = w1.xy, qlo.y = w1.zw, qlo.z = w2.xy, qhi.x = w2.zw, qhi.y = w3.xy, qhi.z = w3.zw
-        const bool nx = r.invd.x < 0.0f, ny = r.invd.y < 0.0f, nz = r.invd.z < 0.0f;
-        const uint32_t nxl = nx ? w2.z : w1.x, nxh = nx ? w2.w : w1.y;
-        const uint32_t fxl = nx ? w1.x : w2.z, fxh = nx ? w1.y : w2.w;
-        const uint32_t nyl = ny ? w3.x : w1.z, nyh = ny ? w3.y : w1.w;
-        const uint32_t fyl = ny ? w1.z : w3.x, fyh = ny ? w1.w : w3.y;
-        const uint32_t nzl = nz ? w3.z : w2.x, nzh = nz ? w3.w : w2.y;
-        const uint32_t fzl = nz ? w2.x : w3.z, fzh = nz ? w2.y : w3.w;
-        uint32_t hit = 0;
-#ifdef __CUDA_ARCH__
-#pragma unroll
-#endif
-        for (int s = 0; s < 8; s++)
-        {
-            const float tnx = fma_hd(byte_to_float(nxl, nxh, s), ax, bnx);
-            const float tny = fma_hd(byte_to_float(nyl, nyh, s), ay, bny);
-            const float tnz = fma_hd(byte_to_float(nzl, nzh, s), az, bnz);
-            const float tfx = fma_hd(byte_to_float(fxl, fxh, s), ax, bfx);
-            const float tfy = fma_hd(byte_to_float(fyl, fyh, s), ay, bfy);
-            const float tfz = fma_hd(byte_to_float(fzl, fzh, s), az, bfz);
-            const float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin));
-            const float tf = fminf(fminf(tfx, tfy), fminf(tfz, tmax));
-            hit |= (tn <= tf ? 1u : 0u) << s;
-        }
-        return hit;
+        const SlabAxis x = slab_axis<true>(dx, sx, r.invd.x, w1.x, w1.y, w2.z, w2.w);
+        const SlabAxis y = slab_axis<false>(dy, sy, r.invd.y, w1.z, w1.w, w3.x, w3.y);
+        const SlabAxis z = slab_axis<false>(dz, sz, r.invd.z, w2.x, w2.y, w3.z, w3.w);
+        uint32_t missed = 0;
+        slab_child<7>(x, y, z, tmin, tmax, missed);
+        slab_child<6>(x, y, z, tmin, tmax, missed);
+        slab_child<5>(x, y, z, tmin, tmax, missed);
+        slab_child<4>(x, y, z, tmin, tmax, missed);
+        slab_child<3>(x, y, z, tmin, tmax, missed);
+        slab_child<2>(x, y, z, tmin, tmax, missed);
+        slab_child<1>(x, y, z, tmin, tmax, missed);
+        slab_child<0>(x, y, z, tmin, tmax, missed);
+        return ~missed & 0xFFu;
     }
 
     // Moller-Trumbore with the reference's determinant cull and inclusive edges

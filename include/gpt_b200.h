@@ -136,9 +136,9 @@ typedef struct gpt_render_settings {
     uint32_t loop_mode;           /* GPT_LOOP_GRAPH (default): the whole frame is one CUDA graph whose conditional WHILE
                                      node repeats the iteration on the device; GPT_LOOP_HOST: the host launches each
                                      iteration and reads the loop condition after it (the reference's structure) */
-    uint32_t trace_occupancy;     /* traversal kernel variant: 0/1 = registers unconstrained, 10 or 12 = that many
-                                     resident 128-thread blocks per SM targeted (fewer registers, more warps) */
-    uint32_t bvh_format;          /* GPT_BVH8_Q8 (default): 8-wide BVH, 8-bit quantised child boxes, 128-B nodes;
+    uint32_t trace_occupancy;     /* traversal kernel variant: 1 = registers unconstrained, 0 or 10 = 9 resident
+                                     128-thread blocks per SM targeted, 12 = 12 (fewer registers, more warps) */
+    uint32_t bvh_format;          /* GPT_BVH8_Q8 (default): 8-wide BVH, 8-bit quantised child boxes, 64-B nodes;
                                      GPT_BVH2_FP32: the binary BVH it is collapsed from, FP32 child boxes, 64-B nodes,
                                      local-memory stack (the plain format; same hits, bit for bit) */
     uint32_t wavefront_layout;    /* GPT_WAVEFRONT_B200 (default): finished slots are regenerated from a bitmap in

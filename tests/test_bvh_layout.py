@@ -37,6 +37,10 @@ def test_block_traversal_equals_the_binary_bvh(gpu_renderer, name, scale, offset
     # scaled rays: origins and lengths follow the scene, directions stay unit vectors
     rays[:, 0:3] = rays[:, 0:3] * np.float32(scale) + np.asarray(offset, dtype=np.float32)
     rays[:, 6] = np.float32(1e-4 * scale)
+    # axis-parallel rays: their clamped reciprocals overflow in the slab tests of large scenes
+    axis = rays[:3001].copy()
+    axis[:, 3:6] = np.repeat(np.concatenate([np.eye(3), -np.eye(3)]), 501, 0)[:3001].astype(np.float32)
+    rays = np.concatenate([rays, axis])
     r = gpu_renderer
     r.upload_scene(s)
     tri, uvt = r.trace_closest_np(rays, pathtracer.BVH2_FP32)

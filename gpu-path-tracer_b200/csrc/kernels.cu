@@ -33,14 +33,14 @@ namespace pt
     }
 
     // Same, grouping lanes by key (queue id); counters[key] is the queue's size.
-    __device__ __forceinline__ uint32_t agg_push_keyed(uint32_t* counters, uint32_t key)
+    __device__ __forceinline__ uint32_t agg_push_keyed(Spread<uint32_t>* counters, uint32_t key)
     {
         const unsigned active = __activemask();
         const unsigned peers = __match_any_sync(active, key);
         const int leader = __ffs(peers) - 1;
         const uint32_t lane = lane_id();
         uint32_t base = 0;
-        if (static_cast<int>(lane) == leader) base = atomicAdd(&counters[key], static_cast<uint32_t>(__popc(peers)));
+        if (static_cast<int>(lane) == leader) base = atomicAdd(&counters[key].v, static_cast<uint32_t>(__popc(peers)));
         base = __shfl_sync(peers, base, leader);
         return base + static_cast<uint32_t>(__popc(peers & ((1u << lane) - 1u)));
     }
@@ -55,12 +55,12 @@ namespace pt
     // Phase timing: thread 0 of every block stamps its start (min) and its end (max).
     __device__ __forceinline__ void phase_begin(Counters* c, int phase)
     {
-        if (c != nullptr && threadIdx.x == 0) atomicMin(&c->tStart[phase], global_ns());
+        if (c != nullptr && threadIdx.x == 0) atomicMin(&c->tStart[phase].v, global_ns());
     }
     __device__ __forceinline__ void phase_end(Counters* c, int phase)
     {
         __syncthreads();
-        if (c != nullptr && threadIdx.x == 0) atomicMax(&c->tEnd[phase], global_ns());
+        if (c != nullptr && threadIdx.x == 0) atomicMax(&c->tEnd[phase].v, global_ns());
     }
 
     __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
@@ -316,20 +316,31 @@ namespace pt
         }
     }
 
-    // A path left its slot: counted for the iteration and recorded for regeneration, in the finished-slot
-    // bitmap (frame renderer) or the regeneration queue (job engine).
+    // A path left its slot: recorded for regeneration, in the finished-slot bitmap or (the reference's
+    // structure) in the regeneration queue. With the bitmap the caller counts: finished_paths().
     __device__ __forceinline__ void path_finished(const Wavefront& wf, Counters* ctr, uint32_t slot)
     {
         if (wf.regenBits != nullptr)
-        {
-            agg_push(&ctr->regenCount);
             atomicOr(&wf.regenBits[slot >> 5], 1u << (slot & 31u));
-        }
         else
         {
-            const uint32_t pos = agg_push(&ctr->regenCount);
+            const uint32_t pos = agg_push(&ctr->regenCount.v);
             wf.regen[pos] = slot;
         }
+    }
+
+    // Paths that ended in this iteration. With the bitmap, shading counts the paths it ends (once per block)
+    // and the paths that hit nothing are the rays in no model's queue, so the closest-hit kernel counts none.
+    __device__ __forceinline__ uint32_t finished_paths(const Wavefront& wf)
+    {
+        const Counters* c = wf.ctr;
+        uint32_t n = c->regenCount.v;
+        if (wf.regenBits != nullptr)
+        {
+            n += c->rayCount[c->cur].v;
+            for (uint32_t m = 0; m < kModelCount; m++) n -= c->matCount[m].v;
+        }
+        return n;
     }
 
     // Work sources of the persistent traversal kernel.
@@ -343,8 +354,8 @@ namespace pt
         static constexpr bool kFixedTmin = true;   // every wavefront ray starts at kMinT
         __device__ uint32_t root(uint32_t tag) const { return scenes ? __ldg(&scenes[tag >> kSlotBits].root) : 0u; }
         __device__ Counters* counters() const { return wf.ctr; }
-        __device__ uint32_t count() const { return wf.ctr->rayCount[wf.ctr->cur]; }
-        __device__ uint32_t* cursor() const { return &wf.ctr->traceCursor; }
+        __device__ uint32_t count() const { return wf.ctr->rayCount[wf.ctr->cur].v; }
+        __device__ uint32_t* cursor() const { return &wf.ctr->traceCursor.v; }
         __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& tag) const
         {
             const uint32_t cur = wf.ctr->cur;
@@ -393,8 +404,8 @@ namespace pt
         static constexpr bool kFixedTmin = true;
         __device__ uint32_t root(uint32_t tag) const { return scenes ? __ldg(&scenes[tag >> kSlotBits].root) : 0u; }
         __device__ Counters* counters() const { return wf.ctr; }
-        __device__ uint32_t count() const { return wf.ctr->shadowCount; }
-        __device__ uint32_t* cursor() const { return &wf.ctr->shadowCursor; }
+        __device__ uint32_t count() const { return wf.ctr->shadowCount.v; }
+        __device__ uint32_t* cursor() const { return &wf.ctr->shadowCursor.v; }
         __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& tag) const
         {
             const float4 a = wf.shO[i], b = wf.shD[i];
@@ -546,8 +557,8 @@ namespace pt
                 // a step adds at most 8 x 255 tests: flush the packed counters well before a field overflows
                 if (ctr != nullptr && (counts & 0x80008000u))
                 {
-                    atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], static_cast<unsigned long long>(counts & 0xFFFFu));
-                    atomicAdd(&ctr->triTests[ANY ? 1 : 0], static_cast<unsigned long long>(counts >> kTestShift));
+                    atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts & 0xFFFFu));
+                    atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts >> kTestShift));
                     counts = 0;
                 }
             }
@@ -562,8 +573,8 @@ namespace pt
             }
             if (lane == 0)
             {
-                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], v);
-                atomicAdd(&ctr->triTests[ANY ? 1 : 0], t);
+                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, v);
+                atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, t);
             }
         }
         phase_end(ctr, Work::kPhase);
@@ -629,15 +640,15 @@ namespace pt
                 }
                 else
                 {
+                    unsigned laneMaskLt;
+                    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(laneMaskLt));
                     uint32_t base = 0;
                     if (lane == 0) base = atomicAdd(work.cursor(), idleCount);
                     base = __shfl_sync(0xFFFFFFFFu, base, 0);
                     if (base >= n) exhausted = true;
+                    const uint32_t i = base + static_cast<uint32_t>(__popc(idle & laneMaskLt));
                     if (over)
                     {
-                        unsigned laneMaskLt;
-                        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(laneMaskLt));
-                        const uint32_t i = base + static_cast<uint32_t>(__popc(idle & laneMaskLt));
                         if (i < n)
                         {
                             float3 o, d;
@@ -672,8 +683,8 @@ namespace pt
             // a step adds at most one visit and 255 tests: flush the packed counters well before a field overflows
             if (ctr != nullptr && (counts & 0x80008000u))
             {
-                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], static_cast<unsigned long long>(counts & 0xFFFFu));
-                atomicAdd(&ctr->triTests[ANY ? 1 : 0], static_cast<unsigned long long>(counts >> kTestShift));
+                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts & 0xFFFFu));
+                atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts >> kTestShift));
                 counts = 0;
             }
         }
@@ -687,8 +698,8 @@ namespace pt
             }
             if (lane == 0)
             {
-                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0], v);
-                atomicAdd(&ctr->triTests[ANY ? 1 : 0], t);
+                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, v);
+                atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, t);
             }
         }
         phase_end(ctr, Work::kPhase);
@@ -839,15 +850,15 @@ namespace pt
         Counters* c = wf.ctr;
         const uint64_t total = job->totalSamples;
         const uint32_t gen = static_cast<uint32_t>(total < pool ? total : pool);
-        c->rayCount[0] = gen;
-        c->rayCount[1] = 0;
+        c->rayCount[0].v = gen;
+        c->rayCount[1].v = 0;
         c->cur = 0;
-        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m] = 0;
-        c->shadowCount = 0;
-        c->regenCount = 0;
-        c->traceCursor = 0;
-        c->shadowCursor = 0;
-        c->regenCursor = 0;
+        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m].v = 0;
+        c->shadowCount.v = 0;
+        c->regenCount.v = 0;
+        c->traceCursor.v = 0;
+        c->shadowCursor.v = 0;
+        c->regenCursor.v = 0;
         c->iteration = 0;
         c->done = gen == 0 ? 1u : 0u;
         c->errorFlags = 0;
@@ -856,21 +867,21 @@ namespace pt
         c->shadowRaysTraced = 0;
         for (int p = 0; p < 4; p++)
         {
-            c->tStart[p] = ~0ull;
-            c->tEnd[p] = 0;
+            c->tStart[p].v = ~0ull;
+            c->tEnd[p].v = 0;
             c->tAccum[p] = 0;
         }
         for (int k = 0; k < 2; k++)
         {
-            c->nodeVisits[k] = 0;
-            c->triTests[k] = 0;
+            c->nodeVisits[k].v = 0;
+            c->triTests[k].v = 0;
         }
     }
 
     __global__ void generate_kernel(Wavefront wf, const JobView* jobPtr)
     {
         const JobView job = *jobPtr;
-        const uint32_t n = wf.ctr->rayCount[0];
+        const uint32_t n = wf.ctr->rayCount[0].v;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
             start_path(job, 0, wf, i, i, 0, i);
         if (wf.regenBits != nullptr)
@@ -892,9 +903,10 @@ namespace pt
         phase_begin(ctr, 3);
         const unsigned long long launched = ctr->launched;
         const unsigned long long remaining = jobPtr->totalSamples - launched;
-        const uint32_t regenerate = static_cast<uint32_t>(remaining < ctr->regenCount ? remaining : ctr->regenCount);
+        const uint32_t ended = finished_paths(wf);
+        const uint32_t regenerate = static_cast<uint32_t>(remaining < ended ? remaining : ended);
         const uint32_t nxt = ctr->cur ^ 1u;
-        const uint32_t base = ctr->rayCount[nxt];
+        const uint32_t base = ctr->rayCount[nxt].v;
         float* out = jobPtr->sampleRadiance;
         const uint32_t words = (wf.capacity + 31u) >> 5;
         const uint32_t tiles = (words + 31u) >> 5;
@@ -916,7 +928,7 @@ namespace pt
             const uint32_t tileTotal = __shfl_sync(0xFFFFFFFFu, incl, 31);
             if (tileTotal == 0) continue;
             uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&ctr->regenCursor, tileTotal);
+            if (lane == 0) first = atomicAdd(&ctr->regenCursor.v, tileTotal);
             first = __shfl_sync(0xFFFFFFFFu, first, 0);
             const uint32_t excl = incl - count;
             // words in groups of kRegenGroup: the finished slots' loads of a group are in flight together
@@ -1404,7 +1416,7 @@ namespace pt
     {
         Counters* ctr = wf.ctr;
         phase_begin(ctr, 1);
-        const uint32_t n = ctr->matCount[MODEL];
+        const uint32_t n = ctr->matCount[MODEL].v;
         const uint32_t cur = ctr->cur;
         const uint32_t nxt = cur ^ 1u;
         const float4* queue = wf.matQ[MODEL];
@@ -1412,7 +1424,7 @@ namespace pt
         for (uint32_t kb = blockIdx.x * blockDim.x; kb < n; kb += gridDim.x * blockDim.x)
         {
             const uint32_t k = kb + threadIdx.x;
-            bool pushRay = false, pushShadow = false;
+            bool pushRay = false, pushShadow = false, pathEnds = false;
             float4 rayOut0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rayOut1 = rayOut0;
             float4 shOut0 = rayOut0, shOut1 = rayOut0, shOut2 = rayOut0;
             if (k < n)
@@ -1564,6 +1576,7 @@ namespace pt
                     shOut1 = make_float4(sh.direction.x, sh.direction.y, sh.direction.z, sh.tMax);
                     shOut2 = make_float4(sh.radiance.x, sh.radiance.y, sh.radiance.z, 0.0f);
                 }
+                pathEnds = terminated;
                 if (terminated) path_finished(wf, ctr, slot);
                 else
                 {
@@ -1580,7 +1593,7 @@ namespace pt
             // the block's extension rays and shadow rays, each grouped by direction octant, take one
             // range of their queue each
             if (threadIdx.x < 16) octCount[threadIdx.x] = 0;
-            __syncthreads();
+            const int ended = __syncthreads_count(pathEnds);
             uint32_t oct = 0, rank = 0, soct = 0, srank = 0;
             if (pushRay)
             {
@@ -1603,8 +1616,9 @@ namespace pt
                     octBase[8 + q] = stotal;
                     stotal += octCount[8 + q];
                 }
-                blockBase[0] = total ? atomicAdd(&ctr->rayCount[nxt], total) : 0u;
-                blockBase[1] = stotal ? atomicAdd(&ctr->shadowCount, stotal) : 0u;
+                blockBase[0] = total ? atomicAdd(&ctr->rayCount[nxt].v, total) : 0u;
+                blockBase[1] = stotal ? atomicAdd(&ctr->shadowCount.v, stotal) : 0u;
+                if (ended && wf.regenBits != nullptr) atomicAdd(&ctr->regenCount.v, static_cast<uint32_t>(ended));
             }
             __syncthreads();
             if (pushRay)
@@ -1632,13 +1646,13 @@ namespace pt
     {
         Counters* ctr = wf.ctr;
         phase_begin(ctr, 3);
-        const uint32_t n = ctr->regenCount;
+        const uint32_t n = ctr->regenCount.v;
         const unsigned long long launched = ctr->launched;
         const unsigned long long total = jobPtr->totalSamples;
         const unsigned long long remaining = total - launched;
         const uint32_t regenerate = static_cast<uint32_t>(remaining < n ? remaining : n);
         const uint32_t nxt = ctr->cur ^ 1u;
-        const uint32_t base = ctr->rayCount[nxt];
+        const uint32_t base = ctr->rayCount[nxt].v;
         float* out = jobPtr->sampleRadiance;
         for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
         {
@@ -1661,34 +1675,35 @@ namespace pt
         const uint32_t cur = c->cur;
         const uint32_t nxt = cur ^ 1u;
         const unsigned long long remaining = jobPtr->totalSamples - c->launched;
-        const uint32_t regenerate = static_cast<uint32_t>(remaining < c->regenCount ? remaining : c->regenCount);
-        const uint32_t next = c->rayCount[nxt] + regenerate;
+        const uint32_t ended = finished_paths(wf);
+        const uint32_t regenerate = static_cast<uint32_t>(remaining < ended ? remaining : ended);
+        const uint32_t next = c->rayCount[nxt].v + regenerate;
         if (c->iteration < wf.logCapacity)
         {
             uint32_t* row = wf.queueLog + static_cast<size_t>(c->iteration) * kQueueLogColumns;
-            row[0] = c->rayCount[cur];
-            for (uint32_t m = 0; m < kModelCount; m++) row[1 + m] = c->matCount[m];
-            row[7] = c->shadowCount;
-            row[8] = c->regenCount;
+            row[0] = c->rayCount[cur].v;
+            for (uint32_t m = 0; m < kModelCount; m++) row[1 + m] = c->matCount[m].v;
+            row[7] = c->shadowCount.v;
+            row[8] = ended;
         }
-        c->raysTraced += c->rayCount[cur];
-        c->shadowRaysTraced += c->shadowCount;
+        c->raysTraced += c->rayCount[cur].v;
+        c->shadowRaysTraced += c->shadowCount.v;
         for (int p = 0; p < 4; p++)
         {
-            if (c->tEnd[p] > c->tStart[p] && c->tStart[p] != ~0ull) c->tAccum[p] += c->tEnd[p] - c->tStart[p];
-            c->tStart[p] = ~0ull;
-            c->tEnd[p] = 0;
+            if (c->tEnd[p].v > c->tStart[p].v && c->tStart[p].v != ~0ull) c->tAccum[p] += c->tEnd[p].v - c->tStart[p].v;
+            c->tStart[p].v = ~0ull;
+            c->tEnd[p].v = 0;
         }
         c->launched += regenerate;
-        c->rayCount[cur] = 0;
-        c->rayCount[nxt] = next;
+        c->rayCount[cur].v = 0;
+        c->rayCount[nxt].v = next;
         c->cur = nxt;
-        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m] = 0;
-        c->shadowCount = 0;
-        c->regenCount = 0;
-        c->traceCursor = 0;
-        c->shadowCursor = 0;
-        c->regenCursor = 0;
+        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m].v = 0;
+        c->shadowCount.v = 0;
+        c->regenCount.v = 0;
+        c->traceCursor.v = 0;
+        c->shadowCursor.v = 0;
+        c->regenCursor.v = 0;
         c->iteration += 1;
         const bool cancelled = wf.cancel != nullptr && *wf.cancel != 0u;
         // Every path ends within depthLimit iterations, so the frame needs at most
@@ -1818,7 +1833,7 @@ namespace pt
         if (blockIdx.x != 0 || threadIdx.x != 0) return;
         Counters* c = wf.ctr;
         *c = Counters{};
-        for (int p = 0; p < 4; p++) c->tStart[p] = ~0ull;
+        for (int p = 0; p < 4; p++) c->tStart[p].v = ~0ull;
         EngineCtl* e = ev.ctl;
         e->freeCount = pool;
         e->launchCount = 0;
@@ -1831,7 +1846,7 @@ namespace pt
     __global__ void plan_kernel(Wavefront wf, EngineView ev)
     {
         EngineCtl* e = ev.ctl;
-        const uint32_t avail = wf.ctr->regenCount + e->freeCount;
+        const uint32_t avail = finished_paths(wf) + e->freeCount;
         uint32_t launch = 0, segments = 0;
         // a job marked kOrderInTurn gets slots only once every marked job before it has launched all
         // its samples (its turn has come), even if an earlier one's pass window holds it back for now
@@ -1931,13 +1946,13 @@ namespace pt
     {
         Counters* ctr = wf.ctr;
         phase_begin(ctr, 3);
-        const uint32_t n = ctr->regenCount;
+        const uint32_t n = finished_paths(wf);
         const EngineCtl* e = ev.ctl;
         const uint32_t launch = e->launchCount;
         const uint32_t freeCount = e->freeCount;
         const uint32_t segmentCount = e->segmentCount;
         const uint32_t nxt = ctr->cur ^ 1u;
-        const uint32_t base = ctr->rayCount[nxt];
+        const uint32_t base = ctr->rayCount[nxt].v;
         const uint32_t words = (wf.capacity + 31u) >> 5;
         const uint32_t tiles = (words + 31u) >> 5;
         const uint32_t lane = lane_id();
@@ -1971,7 +1986,7 @@ namespace pt
             const uint32_t tileTotal = __shfl_sync(0xFFFFFFFFu, incl, 31);
             if (tileTotal == 0) continue;
             uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&ctr->regenCursor, tileTotal);
+            if (lane == 0) first = atomicAdd(&ctr->regenCursor.v, tileTotal);
             first = __shfl_sync(0xFFFFFFFFu, first, 0);
             const uint32_t excl = incl - count;
             // words in groups of kRegenGroup: the finished slots' loads of a group are in flight together
@@ -2107,26 +2122,26 @@ namespace pt
         const uint32_t cur = c->cur;
         const uint32_t nxt = cur ^ 1u;
         const uint32_t launch = e->launchCount;
-        const uint32_t next = c->rayCount[nxt] + launch;
-        c->raysTraced += c->rayCount[cur];
-        c->shadowRaysTraced += c->shadowCount;
+        const uint32_t next = c->rayCount[nxt].v + launch;
+        c->raysTraced += c->rayCount[cur].v;
+        c->shadowRaysTraced += c->shadowCount.v;
         for (int p = 0; p < 4; p++)
         {
-            if (c->tEnd[p] > c->tStart[p] && c->tStart[p] != ~0ull) c->tAccum[p] += c->tEnd[p] - c->tStart[p];
-            c->tStart[p] = ~0ull;
-            c->tEnd[p] = 0;
+            if (c->tEnd[p].v > c->tStart[p].v && c->tStart[p].v != ~0ull) c->tAccum[p] += c->tEnd[p].v - c->tStart[p].v;
+            c->tStart[p].v = ~0ull;
+            c->tEnd[p].v = 0;
         }
-        e->freeCount = e->freeCount + c->regenCount - launch;
+        e->freeCount = e->freeCount + finished_paths(wf) - launch;
         c->launched += launch;
-        c->rayCount[cur] = 0;
-        c->rayCount[nxt] = next;
+        c->rayCount[cur].v = 0;
+        c->rayCount[nxt].v = next;
         c->cur = nxt;
-        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m] = 0;
-        c->shadowCount = 0;
-        c->regenCount = 0;
-        c->traceCursor = 0;
-        c->shadowCursor = 0;
-        c->regenCursor = 0;
+        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m].v = 0;
+        c->shadowCount.v = 0;
+        c->regenCount.v = 0;
+        c->traceCursor.v = 0;
+        c->shadowCursor.v = 0;
+        c->regenCursor.v = 0;
         c->iteration += 1;
         e->launchCount = 0;
         e->segmentCount = 0;

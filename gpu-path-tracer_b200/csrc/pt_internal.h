@@ -222,33 +222,45 @@ namespace pt
         const volatile uint32_t* doorbell;  // host-mapped: nonzero ends the slice after the current iteration
     };
 
+    // A counter that many warps update at once, in a 256-byte line of its own. Atomics on one line are served
+    // one after another by one L2 slice, and a closest-hit warp does about 6 per refill (ray cursor, queue of
+    // each model): with all counters in one 64-byte struct they bound the kernel (spheres-1m frame: refilling
+    // at 4, 8, 12, 16 or 20 idle lanes took 93, 64, 52, 46 and 44 ms of closest-hit time for the same rays).
+    // Spread: 38.7 ms instead of 45.0; Cornell box frame 1.13 ms instead of 2.01. Taking 64 to 256 rays per
+    // cursor atomic on top of it was slower (41.9 to 44.9 ms).
+    template <class T>
+    struct alignas(256) Spread
+    {
+        T v;
+    };
+
     // Device-resident frame control block. One thread (advance kernel) mutates it
     // between the other kernels of an iteration.
     struct Counters
     {
-        uint32_t rayCount[2];
         uint32_t cur;
-        uint32_t matCount[kModelCount];
-        uint32_t shadowCount;
-        uint32_t regenCount;
-        uint32_t traceCursor;
-        uint32_t shadowCursor;
-        uint32_t regenCursor;     // new samples handed out by the bitmap regeneration of the iteration
         uint32_t iteration;
         uint32_t done;
         uint32_t errorFlags;
         unsigned long long launched;
         unsigned long long raysTraced;
         unsigned long long shadowRaysTraced;
-        // Device time of each kernel phase: first-block start and last-block end (%globaltimer, ns)
-        // of the current launch, summed over iterations by the advance kernel.
-        // Phases: 0 closest-hit traversal, 1 shading (all models), 2 shadow traversal, 3 regeneration.
-        unsigned long long tStart[4];
-        unsigned long long tEnd[4];
         unsigned long long tAccum[4];
+        Spread<uint32_t> rayCount[2];
+        Spread<uint32_t> matCount[kModelCount];
+        Spread<uint32_t> shadowCount;
+        Spread<uint32_t> regenCount;      // paths ended by shading (with a regeneration queue: its size, misses included)
+        Spread<uint32_t> traceCursor;
+        Spread<uint32_t> shadowCursor;
+        Spread<uint32_t> regenCursor;     // new samples handed out by the bitmap regeneration of the iteration
+        // Device time of each kernel phase: first-block start and last-block end (%globaltimer, ns)
+        // of the current launch, summed over iterations (tAccum) by the advance kernel.
+        // Phases: 0 closest-hit traversal, 1 shading (all models), 2 shadow traversal, 3 regeneration.
+        Spread<unsigned long long> tStart[4];
+        Spread<unsigned long long> tEnd[4];
         // Traversal work: BVH8 node visits and triangle tests; [0] closest hit, [1] shadow rays.
-        unsigned long long nodeVisits[2];
-        unsigned long long triTests[2];
+        Spread<unsigned long long> nodeVisits[2];
+        Spread<unsigned long long> triTests[2];
     };
 
     struct Wavefront

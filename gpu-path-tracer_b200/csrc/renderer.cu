@@ -708,8 +708,8 @@ namespace pt
                 stats->shadow_rays = ctr.shadowRaysTraced;
                 for (int k = 0; k < 2; k++)
                 {
-                    stats->node_visits[k] = ctr.nodeVisits[k];
-                    stats->triangle_tests[k] = ctr.triTests[k];
+                    stats->node_visits[k] = ctr.nodeVisits[k].v;
+                    stats->triangle_tests[k] = ctr.triTests[k].v;
                 }
                 stats->device_ms = ms;
                 stats->trace_event_ms = traceEventMs;

@@ -85,11 +85,6 @@ namespace pt
         int sp;
     };
 
-    // Traversal work of a lane: node visits in bits 0-15, triangle tests in bits 16-31 (flushed to
-    // the frame counters before either field can overflow).
-    constexpr uint32_t kVisit = 1u;
-    constexpr uint32_t kTestShift = 16;
-
     // Shared-memory slot of one thread: [0] = direction xyz, tag; [1] = hit u, v,
     // triangle | model << 24 (kInvalid while there is no hit), queue index.
     struct ColdSlot
@@ -107,13 +102,13 @@ namespace pt
     // FIXED: the query's tMin is the wavefront's constant kMinT (no register holds it).
     template <bool ANY, bool FIXED>
     __device__ __forceinline__ bool leaf_tests(const SceneView& sc, TraversalState& st, ColdSlot cold, const uint4* tp,
-                                               bool& occluded, uint32_t& work)
+                                               bool& occluded, uint32_t& tests)
     {
         const float tmin = FIXED ? kMinT : st.ray.tmin;
         const float3 d = cold.direction();
         for (;;)
         {
-            work += 1u << kTestShift;
+            tests++;
             uint4 ua, ub;
             ldg8(tp, ua, ub);
             const float4 a = make_float4(__uint_as_float(ua.x), __uint_as_float(ua.y), __uint_as_float(ua.z), __uint_as_float(ua.w));
@@ -187,7 +182,7 @@ namespace pt
     // farther pushed. Stack entries are node indices. Returns false when traversal is over.
     template <bool ANY, bool FIXED>
     __device__ __forceinline__ bool traverse_step_binary(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t* stack, int stackCap,
-                                                         bool& occluded, uint32_t* errorFlags, uint32_t& work)
+                                                         bool& occluded, uint32_t* errorFlags, uint32_t& visits, uint32_t& tests)
     {
         uint32_t node;
         if (st.pending != kInvalid)
@@ -201,7 +196,7 @@ namespace pt
             node = stack[--st.sp];
         }
         const uint4* nw = sc.nodes2[node].w;
-        work += kVisit;
+        visits++;
         const uint4 w0 = ldg4(nw + 0), w1 = ldg4(nw + 1), w2 = ldg4(nw + 2), w3 = ldg4(nw + 3);
         float tn0, tn1;
         const bool h0 = ((w3.z >> 24) & 1u) &&
@@ -212,9 +207,9 @@ namespace pt
                                   __uint_as_float(w2.z), __uint_as_float(w2.w), st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT, tn1);
         const uint32_t leafMask = (w3.z >> 16) & 3u;
         if (h0 && (leafMask & 1u))
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.x].w, occluded, work)) return false;
+            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.x].w, occluded, tests)) return false;
         if (h1 && (leafMask & 2u))
-            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.y].w, occluded, work)) return false;
+            if (!leaf_tests<ANY, FIXED>(sc, st, cold, sc.records[w3.y].w, occluded, tests)) return false;
         const bool in0 = h0 && !(leafMask & 1u), in1 = h1 && !(leafMask & 2u);
         if (in0 && in1)
         {
@@ -247,12 +242,15 @@ namespace pt
     constexpr int kLeafQueue = 2;
     // Leaves are tested once 1 / kLeafShare of the warp's busy lanes have some waiting.
     constexpr int kLeafShare = 3;
+    // Node visits of a step, between which the warp looks neither at its leaves nor for idle lanes.
+    constexpr int kClosestVisits = 2;
+    constexpr int kAnyVisits = 3;
 
     // One node visit of the BVH8. leaves: group of leaf children waiting for their tests (block << 8 |
     // slots in traversal order, 0 = none), waiting: further groups in queue[].
     template <bool FIXED>
     __device__ __forceinline__ void visit_node(const SceneView& sc, TraversalState& st, uint32_t* stack, uint32_t stride, int stackCap,
-                                               uint32_t& leaves, int& waiting, uint32_t* queue, uint32_t* errorFlags, uint32_t& work)
+                                               uint32_t& leaves, int& waiting, uint32_t* queue, uint32_t* errorFlags, uint32_t& visits)
     {
         uint32_t* top = stack + static_cast<uint32_t>(st.sp - 1) * stride;
         const uint32_t entry = *top;
@@ -261,11 +259,11 @@ namespace pt
         else *top = entry & (entry - 1u);
         const uint32_t slot = static_cast<uint32_t>(__ffs(m) - 1) ^ st.ray.oct;
         const uint4* nw = sc.records[static_cast<size_t>(entry >> 8) * kBlockRecords + slot].w;
-        work += kVisit;
+        visits++;
         uint4 w0, w1, w2, w3;
         ldg8(nw, w0, w1);
         ldg8(nw + 2, w2, w3);
-        const uint32_t hitSlots = intersect_children(w0, w1, w2, w3, st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT);
+        const uint32_t hitSlots = intersect_children<FIXED>(w0, w1, w2, w3, st.ray, FIXED ? kMinT : st.ray.tmin, st.hitT);
         const uint32_t inner = hitSlots & w0.x & 0xFFu;
         const uint32_t both = permute_masks(inner | ((hitSlots & ~w0.x) << 8), st.ray.oct);
         const uint32_t block = w0.w & ~0xFFu;
@@ -296,7 +294,7 @@ namespace pt
     // Tests the next triangle of the lane's waiting leaves. An any-hit query that finds an occluder ends.
     template <bool ANY, bool FIXED>
     __device__ __forceinline__ void test_leaf(const SceneView& sc, TraversalState& st, ColdSlot cold, uint32_t& leaves, int& waiting,
-                                              const uint32_t* queue, uint32_t stride, uint32_t& work)
+                                              const uint32_t* queue, uint32_t stride, uint32_t& tests)
     {
         const uint32_t slot = static_cast<uint32_t>(__ffs(leaves & 0xFFu) - 1) ^ st.ray.oct;
         const uint4* tp = sc.records[static_cast<size_t>(leaves >> 8) * kBlockRecords + slot].w;
@@ -307,7 +305,7 @@ namespace pt
             if (waiting > 0) leaves = queue[static_cast<uint32_t>(--waiting) * stride];
         }
         bool occluded = false;
-        if (!leaf_tests<ANY, FIXED>(sc, st, cold, tp, occluded, work))
+        if (!leaf_tests<ANY, FIXED>(sc, st, cold, tp, occluded, tests))
         {
             cold.p[1].z = __uint_as_float(0u);
             st.sp = 0;
@@ -487,7 +485,7 @@ namespace pt
         // entries a ray may push: the stack's capacity, or the caller's smaller bound (pushes beyond it
         // are refused and reported as an overflow)
         const int cap = (work.stackCap > 0 && work.stackCap < STACK) ? work.stackCap : STACK;
-        uint32_t counts = 0;  // node visits | triangle tests << 16
+        uint32_t visits = 0, tests = 0;  // traversal work of the lane
         const uint32_t lane = lane_id();
         TraversalState st;
         bool active = false;
@@ -539,7 +537,7 @@ namespace pt
 #pragma unroll 1
                 for (int k = 0; k < 4 && more; k++)
                 {
-                    more = traverse_step_binary<ANY, Work::kFixedTmin>(work.sc, st, cold, stack, cap, occluded, errorFlags, counts);
+                    more = traverse_step_binary<ANY, Work::kFixedTmin>(work.sc, st, cold, stack, cap, occluded, errorFlags, visits, tests);
                 }
                 if (!more)
                 {
@@ -554,18 +552,11 @@ namespace pt
                     work.finish(__float_as_uint(c1.w), __float_as_uint(c0.w), h, occluded, st.ray.o, make_float3(c0.x, c0.y, c0.z));
                     active = false;
                 }
-                // a step adds at most 8 x 255 tests: flush the packed counters well before a field overflows
-                if (ctr != nullptr && (counts & 0x80008000u))
-                {
-                    atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts & 0xFFFFu));
-                    atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts >> kTestShift));
-                    counts = 0;
-                }
             }
         }
         if (ctr != nullptr)
         {
-            unsigned long long v = counts & 0xFFFFu, t = counts >> kTestShift;
+            unsigned long long v = visits, t = tests;
             for (int o = 16; o > 0; o >>= 1)
             {
                 v += __shfl_down_sync(0xFFFFFFFFu, v, o);
@@ -581,7 +572,7 @@ namespace pt
     }
 
 
-    // The same for the BVH8, with the warp's lanes in step: each step visits one node per lane, then tests
+    // The same for the BVH8, with the warp's lanes in step: each step visits a few nodes per lane, then tests
     // one triangle per lane if enough lanes hold leaves (kLeafShare), and goes on testing while more than
     // half of the busy lanes do. A node visit rarely enters leaves in more than a few lanes (0.34 tests per
     // visit on spheres-1m), so testing them at once ran the triangle test for 7, then 2, then 1 lane of the
@@ -591,6 +582,8 @@ namespace pt
     // 92.7 ms; a share of 1/2, 1/4 or 1/8 measured 92.5, 91.8, 92.1 (before the loop), a fixed 6, 16 or 22
     // lanes 92.2, 97.8, 124 and 1.7 times the time of small batches, whose warps are seldom full. Without
     // the loop the Cornell box, with its 1.3 tests per visit, took 5.06 instead of 4.77 ms.
+    // Two visits per step (three for any-hit rays) halve the votes: 80.6 -> 77.3 ms with the floor of the box
+    // test and the work counters in registers of their own; three visits for closest hits measured the same.
     // Finished rays stay in their lanes until the next refill, which retires them together.
     // Traversal stack: STACK entries per thread, entry = child block << 8 | child mask.
     // Shared memory: [cold slots: 2 x float4 per thread][stack: STACK words per thread][kLeafQueue words per thread].
@@ -606,7 +599,7 @@ namespace pt
         phase_begin(ctr, Work::kPhase);
         const uint32_t n = work.count();
         const int cap = (work.stackCap > 0 && work.stackCap < STACK) ? work.stackCap : STACK;
-        uint32_t counts = 0;  // node visits | triangle tests << 16
+        uint32_t visits = 0, tests = 0;  // traversal work of the lane
         const uint32_t lane = lane_id();
         TraversalState st;
         st.sp = 0;
@@ -621,6 +614,9 @@ namespace pt
             const uint32_t idleCount = static_cast<uint32_t>(__popc(idle));
             if (idleCount >= refill || idle == 0xFFFFFFFFu)
             {
+                // the cursor's atomic is in flight while the finished rays are retired
+                uint32_t base = 0;
+                if (!exhausted && lane == 0) base = atomicAdd(work.cursor(), idleCount);
                 if (over && active)
                 {
                     const float4 c0 = cold.p[0], c1 = cold.p[1];
@@ -642,8 +638,6 @@ namespace pt
                 {
                     unsigned laneMaskLt;
                     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(laneMaskLt));
-                    uint32_t base = 0;
-                    if (lane == 0) base = atomicAdd(work.cursor(), idleCount);
                     base = __shfl_sync(0xFFFFFFFFu, base, 0);
                     if (base >= n) exhausted = true;
                     const uint32_t i = base + static_cast<uint32_t>(__popc(idle & laneMaskLt));
@@ -668,29 +662,24 @@ namespace pt
                     continue;
                 }
             }
-            if (st.sp > 0 && waiting < kLeafQueue)
-                visit_node<Work::kFixedTmin>(work.sc, st, stack, stride, cap, leaves, waiting, queue, errorFlags, counts);
+#pragma unroll 1
+            for (int k = 0; k < (ANY ? kAnyVisits : kClosestVisits); k++)
+                if (st.sp > 0 && waiting < kLeafQueue)
+                    visit_node<Work::kFixedTmin>(work.sc, st, stack, stride, cap, leaves, waiting, queue, errorFlags, visits);
             unsigned holding = __ballot_sync(0xFFFFFFFFu, leaves != 0);
             const unsigned busy = holding | __ballot_sync(0xFFFFFFFFu, st.sp > 0);
             if (__popc(holding) * kLeafShare >= __popc(busy))
             {
                 do
                 {
-                    if (leaves != 0) test_leaf<ANY, Work::kFixedTmin>(work.sc, st, cold, leaves, waiting, queue, stride, counts);
+                    if (leaves != 0) test_leaf<ANY, Work::kFixedTmin>(work.sc, st, cold, leaves, waiting, queue, stride, tests);
                     holding = __ballot_sync(0xFFFFFFFFu, leaves != 0);
                 } while (__popc(holding) * 2 > __popc(busy));
-            }
-            // a step adds at most one visit and 255 tests: flush the packed counters well before a field overflows
-            if (ctr != nullptr && (counts & 0x80008000u))
-            {
-                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts & 0xFFFFu));
-                atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, static_cast<unsigned long long>(counts >> kTestShift));
-                counts = 0;
             }
         }
         if (ctr != nullptr)
         {
-            unsigned long long v = counts & 0xFFFFu, t = counts >> kTestShift;
+            unsigned long long v = visits, t = tests;
             for (int o = 16; o > 0; o >>= 1)
             {
                 v += __shfl_down_sync(0xFFFFFFFFu, v, o);

@@ -106,22 +106,28 @@ namespace pt
         return r;
     }
 
-    // Shifts 1 into `missed` when the ray misses child S, else 0.
-    template <int S>
+    // Shifts 1 into `missed` when the ray misses child S, else 0. FIXED (tmin close to 0): the entry distance is
+    // clamped to 0 by the three-input integer maximum with a zero floor (the bits of floats that are not negative
+    // order like integers; NaNs stay NaNs or are ignored), which takes one operation less than a clamp to tmin.
+    template <int S, bool FIXED>
     __device__ __forceinline__ void slab_child(const SlabAxis& x, const SlabAxis& y, const SlabAxis& z, float tmin, float tmax, uint32_t& missed)
     {
-        const float tn = fmaxf(max3f(slab_plane<S, true>(x.nearLo, x.nearHi, x.a, x.near), slab_plane<S, false>(y.nearLo, y.nearHi, y.a, y.near),
-                                     slab_plane<S, false>(z.nearLo, z.nearHi, z.a, z.near)),
-                               tmin);
-        const float tf = fminf(min3f(slab_plane<S, true>(x.farLo, x.farHi, x.a, x.far), slab_plane<S, false>(y.farLo, y.farHi, y.a, y.far),
-                                     slab_plane<S, false>(z.farLo, z.farHi, z.a, z.far)),
-                               tmax);
+        const float nx = slab_plane<S, true>(x.nearLo, x.nearHi, x.a, x.near);
+        const float ny = slab_plane<S, false>(y.nearLo, y.nearHi, y.a, y.near);
+        const float nz = slab_plane<S, false>(z.nearLo, z.nearHi, z.a, z.near);
+        const float fx = slab_plane<S, true>(x.farLo, x.farHi, x.a, x.far);
+        const float fy = slab_plane<S, false>(y.farLo, y.farHi, y.a, y.far);
+        const float fz = slab_plane<S, false>(z.farLo, z.farHi, z.a, z.far);
+        const float tn = FIXED ? __int_as_float(__vimax3_s32_relu(__float_as_int(nx), __float_as_int(ny), __float_as_int(nz)))
+                               : fmaxf(max3f(nx, ny, nz), tmin);
+        const float tf = fminf(min3f(fx, fy, fz), tmax);
         missed = __funnelshift_l(__float_as_uint(tf - tn), missed, 1);
     }
 
     // Slab test of the 8 quantised children against [tmin, tmax], conservative for every child box (a box the
     // exact arithmetic would hit is never culled). Returns the hit mask in slot order. Empty slots hold inverted
     // boxes and are almost always culled; one that passes is a record of zeros, which no ray hits.
+    template <bool FIXED>
     __device__ __forceinline__ uint32_t intersect_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, float tmin, float tmax)
     {
         // unit = 2^(u - 127) is 2^-8 of the origin's grid (the low byte of a word is masked, so it holds
@@ -139,14 +145,14 @@ namespace pt
         const SlabAxis y = slab_axis<false>(dy, sy, r.invd.y, w1.z, w1.w, w3.x, w3.y);
         const SlabAxis z = slab_axis<false>(dz, sz, r.invd.z, w2.x, w2.y, w3.z, w3.w);
         uint32_t missed = 0;
-        slab_child<7>(x, y, z, tmin, tmax, missed);
-        slab_child<6>(x, y, z, tmin, tmax, missed);
-        slab_child<5>(x, y, z, tmin, tmax, missed);
-        slab_child<4>(x, y, z, tmin, tmax, missed);
-        slab_child<3>(x, y, z, tmin, tmax, missed);
-        slab_child<2>(x, y, z, tmin, tmax, missed);
-        slab_child<1>(x, y, z, tmin, tmax, missed);
-        slab_child<0>(x, y, z, tmin, tmax, missed);
+        slab_child<7, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<6, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<5, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<4, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<3, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<2, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<1, FIXED>(x, y, z, tmin, tmax, missed);
+        slab_child<0, FIXED>(x, y, z, tmin, tmax, missed);
         return ~missed & 0xFFu;
     }
 

@@ -57,6 +57,8 @@ namespace pt
         cudaStream_t shadeStreams[kModelCount];
     };
 
+    constexpr int kBatchOccupancy = 10;  // traversal variant of ray batches
+
     int trace_grid_blocks(int device, int threads, uint32_t depth, int occupancy, uint32_t bvhFormat = kBvh8Quantised);
     cudaError_t launch_engine_init(const Wavefront& wf, const EngineView& ev, uint32_t pool, cudaStream_t stream);
     cudaError_t launch_engine_iteration(const EngineLaunch& launch, cudaStream_t stream);

@@ -837,7 +837,7 @@ namespace pt
             PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(cursor, 0, 8, st));
             const SceneView sv = scene_->view();
             if (bvh == kBvh2Fp32 && !sv.nodes2) return Status::Err(GPT_ERR_STATE, "The scene has no binary BVH");
-            const int blocks = trace_grid_blocks(device_, 128, sv.depth, 1, bvh);
+            const int blocks = trace_grid_blocks(device_, 128, sv.depth, kBatchOccupancy, bvh);
             PT_CUDA("intersect", launch_batch_trace(sv, 0u, rays, n, cursor, tri, uvt, occ, blocks, 128, cursor + 1, st, bvh));
             uint32_t err = 0;
             PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&err, cursor + 1, 4, cudaMemcpyDeviceToHost, st));

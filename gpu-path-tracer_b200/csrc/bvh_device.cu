@@ -10,7 +10,9 @@
 //    kPlocRadius positions whose merged box has the smallest surface area (the nearer position wins a
 //    tie), mutual nearest neighbours merge, and the survivors are compacted in order by prefix sums,
 //    until one cluster is left. The nodes of one round get consecutive indices after those of the
-//    rounds before, so every node has a larger index than its children.
+//    rounds before, so every node has a larger index than its children. The cluster count stays on the
+//    device, and the host reads it every kRoundsPerSync rounds only; the last rounds, with at most
+//    kTailClusters clusters, run in one block.
 // 4. The collapse's cost table (Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on
 //    GPUs Through Compressed Wide BVHs", HPG 2017), bottom-up one round of nodes at a time.
 // 5. Wide nodes level by level from the root: each collects its children from the cost table,
@@ -36,6 +38,8 @@ namespace pt
     {
         constexpr int kPlocRadius = 16;
         constexpr int kPlocBlock = 256;
+        constexpr uint32_t kTailClusters = 1024;  // clusters (and threads) of the one-block rounds
+        constexpr int kRoundsPerSync = 3;         // grids are sized by the last count read, at most 8 times too large then
         constexpr float kCollapseNodeCost = 2.0f;  // a wide-node visit against one triangle test (bvh8.cpp)
         constexpr int kCollectStack = 24;
         constexpr uint32_t kBuildErrExponent = 1u;  // quantisation exponent overflow
@@ -164,9 +168,18 @@ namespace pt
         }
 
         // Nearest neighbour of every cluster within kPlocRadius positions (surface area of the merged box).
-        __global__ void __launch_bounds__(kPlocBlock) ploc_nearest_kernel(const uint32_t* clusters, uint32_t m, const float4* lo, const float4* hi,
-                                                                          uint32_t* nn)
+        // Clustering state on the device: clusters left, next node index, rounds done (roundEnd[r]: first node
+        // index behind round r - 1), and whether a round merged nothing.
+        struct PlocState
         {
+            uint32_t clusters, nodes, rounds, stalled;
+        };
+
+        __global__ void __launch_bounds__(kPlocBlock) ploc_nearest_kernel(const uint32_t* clusters, const PlocState* state, const float4* lo,
+                                                                          const float4* hi, uint32_t* nn)
+        {
+            const uint32_t m = state->clusters;
+            if (blockIdx.x * kPlocBlock >= m) return;
             __shared__ float4 sLo[kPlocBlock + 2 * kPlocRadius], sHi[kPlocBlock + 2 * kPlocRadius];
             const int start = static_cast<int>(blockIdx.x) * kPlocBlock - kPlocRadius;
             for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock)
@@ -201,44 +214,165 @@ namespace pt
             nn[i] = static_cast<uint32_t>(bj);
         }
 
-        // merge[i]: cluster i merges with its neighbour into a new node (mutual pair, i the smaller);
-        // keep[i]: a cluster survives at position i (unpaired, or the smaller of a pair). Entry m is 0,
-        // so the exclusive sums over m + 1 entries end with the totals.
-        __global__ void ploc_flags_kernel(const uint32_t* nn, uint32_t m, uint32_t* merge, uint32_t* keep)
+        // flags[i], low word: cluster i merges with its neighbour into a new node (mutual pair, i the smaller);
+        // high word: a cluster survives at position i (unpaired, or the smaller of a pair). Entries from the
+        // cluster count on are 0, so the exclusive sums at the count are the totals.
+        __global__ void ploc_flags_kernel(const uint32_t* nn, const PlocState* state, uint32_t entries, unsigned long long* flags)
         {
-            for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= m; i += gridDim.x * blockDim.x)
+            const uint32_t m = state->clusters;
+            for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < entries; i += gridDim.x * blockDim.x)
             {
-                if (i == m)
+                unsigned long long f = 0;
+                if (i < m)
                 {
-                    merge[i] = 0;
-                    keep[i] = 0;
-                    continue;
+                    const uint32_t j = nn[i];
+                    const bool mutual = nn[j] == i;
+                    f = (mutual && i < j ? 1ull : 0ull) | (mutual && i > j ? 0ull : 1ull << 32);
                 }
-                const uint32_t j = nn[i];
-                const bool mutual = nn[j] == i;
-                merge[i] = mutual && i < j ? 1u : 0u;
-                keep[i] = mutual && i > j ? 0u : 1u;
+                flags[i] = f;
             }
         }
 
-        __global__ void ploc_merge_kernel(const uint32_t* clusters, uint32_t m, const uint32_t* nn, const uint32_t* merge, const uint32_t* mergePos,
-                                          const uint32_t* keep, const uint32_t* keepPos, uint32_t nodeBase, float4* lo, float4* hi, uint2* child,
-                                          uint32_t* next)
+        __global__ void ploc_merge_kernel(const uint32_t* clusters, const PlocState* state, const uint32_t* nn, const unsigned long long* flags,
+                                          const unsigned long long* positions, float4* lo, float4* hi, uint2* child, uint32_t* next)
         {
+            const uint32_t m = state->clusters, nodeBase = state->nodes;
             for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
             {
-                if (!keep[i]) continue;
+                const unsigned long long f = flags[i], at = positions[i];
+                if ((f >> 32) == 0) continue;
                 uint32_t id = clusters[i];
-                if (merge[i])
+                if (f & 1u)
                 {
                     const uint32_t other = clusters[nn[i]];
-                    const uint32_t fresh = nodeBase + mergePos[i];
+                    const uint32_t fresh = nodeBase + static_cast<uint32_t>(at);
                     child[fresh] = make_uint2(id, other);
                     lo[fresh] = fmin4(lo[id], lo[other]);
                     hi[fresh] = fmax4(hi[id], hi[other]);
                     id = fresh;
                 }
-                next[keepPos[i]] = id;
+                next[at >> 32] = id;
+            }
+        }
+
+        __global__ void ploc_advance_kernel(PlocState* state, const unsigned long long* positions, uint32_t* roundEnd)
+        {
+            const unsigned long long totals = positions[state->clusters];
+            const uint32_t merged = static_cast<uint32_t>(totals), kept = static_cast<uint32_t>(totals >> 32);
+            if (merged == 0 || kept != state->clusters - merged)
+            {
+                state->stalled = 1;
+                return;
+            }
+            state->nodes += merged;
+            state->clusters = kept;
+            roundEnd[++state->rounds] = state->nodes;
+        }
+
+        // The rounds from at most kTailClusters clusters on, in one block: the same rounds (and so the same
+        // nodes), with the clusters' boxes in shared memory. Half of a build's rounds have this few clusters, and
+        // as launches with a read of the count they took about 70 us each.
+        __global__ void __launch_bounds__(kTailClusters) ploc_tail_kernel(const uint32_t* clusters, PlocState* state, float4* lo, float4* hi,
+                                                                          uint2* child, uint32_t* roundEnd)
+        {
+            extern __shared__ float4 boxes[];
+            float4* sLo = boxes;
+            float4* sHi = boxes + kTailClusters;
+            __shared__ uint32_t sNear[kTailClusters], sId[kTailClusters], warpMerged[32], warpKept[32];
+            const uint32_t i = threadIdx.x, lane = i & 31u, warp = i >> 5;
+            uint32_t m = state->clusters, nodes = state->nodes, rounds = state->rounds;
+            uint32_t id = 0;
+            float4 myLo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), myHi = myLo;
+            if (i < m)
+            {
+                id = clusters[i];
+                myLo = lo[id];
+                myHi = hi[id];
+            }
+            while (m > 1)
+            {
+                sLo[i] = myLo;
+                sHi[i] = myHi;
+                sId[i] = id;
+                __syncthreads();
+                uint32_t bj = i == 0 ? 1u : i - 1u;
+                if (i < m)
+                {
+                    const uint32_t jLo = i < kPlocRadius ? 0u : i - kPlocRadius;
+                    const uint32_t jHi = i + kPlocRadius > m - 1u ? m - 1u : i + kPlocRadius;
+                    float best = FLT_MAX;
+                    for (uint32_t j = jLo; j <= jHi; j++)
+                    {
+                        if (j == i) continue;
+                        const float a = box_area(fmin4(myLo, sLo[j]), fmax4(myHi, sHi[j]));
+                        if (a < best)
+                        {
+                            best = a;
+                            bj = j;
+                        }
+                    }
+                    sNear[i] = bj;
+                }
+                __syncthreads();
+                const bool mutual = i < m && sNear[bj] == i;
+                const bool merges = mutual && i < bj, keeps = i < m && !(mutual && i > bj);
+                const unsigned mergedMask = __ballot_sync(0xFFFFFFFFu, merges), keptMask = __ballot_sync(0xFFFFFFFFu, keeps);
+                if (lane == 0)
+                {
+                    warpMerged[warp] = static_cast<uint32_t>(__popc(mergedMask));
+                    warpKept[warp] = static_cast<uint32_t>(__popc(keptMask));
+                }
+                __syncthreads();
+                uint32_t mergedBefore = 0, keptBefore = 0, merged = 0, kept = 0;
+                for (uint32_t w = 0; w < kTailClusters / 32; w++)
+                {
+                    mergedBefore += w < warp ? warpMerged[w] : 0u;
+                    keptBefore += w < warp ? warpKept[w] : 0u;
+                    merged += warpMerged[w];
+                    kept += warpKept[w];
+                }
+                if (merged == 0 || kept != m - merged)
+                {
+                    if (i == 0) state->stalled = 1;
+                    return;
+                }
+                const unsigned below = (1u << lane) - 1u;
+                if (merges)
+                {
+                    const uint32_t fresh = nodes + mergedBefore + static_cast<uint32_t>(__popc(mergedMask & below));
+                    child[fresh] = make_uint2(id, sId[bj]);
+                    myLo = fmin4(myLo, sLo[bj]);
+                    myHi = fmax4(myHi, sHi[bj]);
+                    lo[fresh] = myLo;
+                    hi[fresh] = myHi;
+                    id = fresh;
+                }
+                __syncthreads();
+                if (keeps)
+                {
+                    const uint32_t at = keptBefore + static_cast<uint32_t>(__popc(keptMask & below));
+                    sId[at] = id;
+                    sLo[at] = myLo;
+                    sHi[at] = myHi;
+                }
+                __syncthreads();
+                m = kept;
+                nodes += merged;
+                rounds++;
+                if (i == 0) roundEnd[rounds] = nodes;
+                if (i < m)
+                {
+                    id = sId[i];
+                    myLo = sLo[i];
+                    myHi = sHi[i];
+                }
+                __syncthreads();
+            }
+            if (i == 0)
+            {
+                state->clusters = m;
+                state->nodes = nodes;
+                state->rounds = rounds;
             }
         }
 
@@ -257,10 +391,8 @@ namespace pt
             }
         }
 
-        __global__ void collapse_node_kernel(uint32_t first, uint32_t end, const float4* lo, const float4* hi, const uint2* child, float* cost,
-                                             uint8_t* how, uint8_t* split)
+        __device__ void collapse_node(uint32_t i, const float4* lo, const float4* hi, const uint2* child, float* cost, uint8_t* how, uint8_t* split)
         {
-            for (uint32_t i = first + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x)
             {
                 const float A = box_area(lo[i], hi[i]);
                 const uint2 c = child[i];
@@ -310,6 +442,25 @@ namespace pt
                     cost[static_cast<size_t>(i) * 8 + k] = C[k];
                     how[static_cast<size_t>(i) * 8 + k] = H[k];
                 }
+            }
+        }
+
+        __global__ void collapse_node_kernel(uint32_t first, uint32_t end, const float4* lo, const float4* hi, const uint2* child, float* cost,
+                                             uint8_t* how, uint8_t* split)
+        {
+            for (uint32_t i = first + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x)
+                collapse_node(i, lo, hi, child, cost, how, split);
+        }
+
+        // Rounds [firstRound, endRound) by one block, which is enough for their few nodes.
+        __global__ void collapse_tail_kernel(const uint32_t* roundEnd, uint32_t firstRound, uint32_t endRound, const float4* lo, const float4* hi,
+                                             const uint2* child, float* cost, uint8_t* how, uint8_t* split)
+        {
+            for (uint32_t r = firstRound; r < endRound; r++)
+            {
+                const uint32_t end = roundEnd[r + 1];
+                for (uint32_t i = roundEnd[r] + threadIdx.x; i < end; i += blockDim.x) collapse_node(i, lo, hi, child, cost, how, split);
+                __syncthreads();
             }
         }
 
@@ -627,133 +778,144 @@ namespace pt
         if (n == 0) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "BVH build failed: scene has no triangles");
         if (n > kMaxTriangles) return Status::Err(GPT_ERR_CAPACITY, "BVH build failed: scene has more than 2^24 triangles");
         const uint32_t nodes = 2 * n - 1;
-        DeviceBuffer triLo, triHi, cent, partLo, partHi, keys, keysSorted, values, sorted, lo, hi, child, clustersA, clustersB, nn, merge, mergePos, keep,
-            keepPos, cost, how, split, levelA, levelB, counter, errorFlags, temp, wide, headerRecord, nodeMasks, leafRecord;
-        const uint32_t parts = grid_for(n, 256, 1024);
-        PT_TRY(triLo.allocate(size_t(n) * 16));
-        PT_TRY(triHi.allocate(size_t(n) * 16));
-        PT_TRY(cent.allocate(size_t(n) * 16));
-        PT_TRY(partLo.allocate(size_t(parts) * 16));
-        PT_TRY(partHi.allocate(size_t(parts) * 16));
-        PT_TRY(keys.allocate(size_t(n) * 4));
-        PT_TRY(keysSorted.allocate(size_t(n) * 4));
-        PT_TRY(values.allocate(size_t(n) * 4));
-        PT_TRY(sorted.allocate(size_t(n) * 4));
-        PT_TRY(lo.allocate(size_t(nodes) * 16));
-        PT_TRY(hi.allocate(size_t(nodes) * 16));
-        PT_TRY(child.allocate(size_t(nodes) * 8));
-        PT_TRY(clustersA.allocate(size_t(n) * 4));
-        PT_TRY(clustersB.allocate(size_t(n) * 4));
-        PT_TRY(nn.allocate(size_t(n) * 4));
-        PT_TRY(merge.allocate(size_t(n + 1) * 4));
-        PT_TRY(mergePos.allocate(size_t(n + 1) * 4));
-        PT_TRY(keep.allocate(size_t(n + 1) * 4));
-        PT_TRY(keepPos.allocate(size_t(n + 1) * 4));
-        PT_TRY(cost.allocate(size_t(nodes) * 8 * 4));
-        PT_TRY(how.allocate(size_t(nodes) * 8));
-        PT_TRY(split.allocate(size_t(nodes)));
-        PT_TRY(levelA.allocate(size_t(n) * 8));
-        PT_TRY(levelB.allocate(size_t(n) * 8));
-        PT_TRY(counter.allocate(16));
-        PT_TRY(errorFlags.allocate(16));
-        // at most one wide node per binary inner node (one for n = 1)
-        PT_TRY(wide.allocate(size_t(n) * sizeof(Record8)));
-        PT_TRY(headerRecord.allocate(size_t(n) * 4));
-        PT_TRY(nodeMasks.allocate(size_t(n) * 4));
-        PT_TRY(leafRecord.allocate(size_t(n) * 4));
+        float4 *triLo, *triHi, *cent, *partLo, *partHi, *lo, *hi;
+        uint32_t *keys, *keysSorted, *values, *sorted, *clustersA, *clustersB, *nn, *roundEnd, *counter, *errorFlags, *headerRecord, *nodeMasks, *leafRecord;
+        unsigned long long *flags, *ranks;
+        uint2 *child, *levelA, *levelB;
+        float* cost;
+        uint8_t *how, *split;
+        char* temp;
+        Record8* wide;
+        PlocState* state;
         size_t sortBytes = 0, scanBytes = 0;
-        PT_CUDA("cub::DeviceRadixSort::SortPairs", cub::DeviceRadixSort::SortPairs(nullptr, sortBytes, keys.get<uint32_t>(), keysSorted.get<uint32_t>(),
-                                                                                 values.get<uint32_t>(), sorted.get<uint32_t>(), static_cast<int>(n), 0, 30, s));
-        PT_CUDA("cub::DeviceScan::ExclusiveSum", cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, merge.get<uint32_t>(), mergePos.get<uint32_t>(),
-                                                                              static_cast<int>(n + 1), s));
-        PT_TRY(temp.allocate(sortBytes > scanBytes ? sortBytes : scanBytes));
-        PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(errorFlags.get<void>(), 0, 16, s));
+        PT_CUDA("cub::DeviceRadixSort::SortPairs", cub::DeviceRadixSort::SortPairs(nullptr, sortBytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+                                                                                 static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), static_cast<int>(n), 0, 30, s));
+        PT_CUDA("cub::DeviceScan::ExclusiveSum", cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, static_cast<unsigned long long*>(nullptr),
+                                                                              static_cast<unsigned long long*>(nullptr), static_cast<int>(n + 1), s));
+        const size_t tempBytes = sortBytes > scanBytes ? sortBytes : scanBytes;
+        const uint32_t parts = grid_for(n, 256, 1024);
+        // One allocation instead of 30 and their frees, three rounds per read of the count and one block for the
+        // last rounds: 22.5 -> 4.9 ms for 1.3M triangles (34 rounds with more than kTailClusters clusters).
+        DeviceArena arena;
+        arena.add(triLo, n);
+        arena.add(triHi, n);
+        arena.add(cent, n);
+        arena.add(partLo, parts);
+        arena.add(partHi, parts);
+        arena.add(keys, n);
+        arena.add(keysSorted, n);
+        arena.add(values, n);
+        arena.add(sorted, n);
+        arena.add(lo, nodes);
+        arena.add(hi, nodes);
+        arena.add(child, nodes);
+        arena.add(clustersA, n);
+        arena.add(clustersB, n);
+        arena.add(nn, n);
+        arena.add(flags, size_t(n) + 1);
+        arena.add(ranks, size_t(n) + 1);
+        arena.add(roundEnd, size_t(n) + 1);  // every round merges at least one pair
+        arena.add(cost, size_t(nodes) * 8);
+        arena.add(how, size_t(nodes) * 8);
+        arena.add(split, nodes);
+        arena.add(levelA, n);
+        arena.add(levelB, n);
+        arena.add(counter, 4);
+        arena.add(errorFlags, 4);
+        arena.add(state, 1);
+        arena.add(wide, n);  // at most one wide node per binary inner node (one for n = 1)
+        arena.add(headerRecord, n);
+        arena.add(nodeMasks, n);
+        arena.add(leafRecord, n);
+        arena.add(temp, tempBytes);
+        PT_TRY(arena.allocate());
+        PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(errorFlags, 0, 16, s));
 
         // 1-2: boxes, centroids, Morton order
-        triangle_boxes_kernel<<<parts, 256, 0, s>>>(positions, n, triLo.get<float4>(), triHi.get<float4>(), cent.get<float4>(), partLo.get<float4>(),
-                                                    partHi.get<float4>());
+        triangle_boxes_kernel<<<parts, 256, 0, s>>>(positions, n, triLo, triHi, cent, partLo, partHi);
         PT_CUDA("triangle boxes", cudaGetLastError());
-        bounds_final_kernel<<<1, 256, 0, s>>>(partLo.get<float4>(), partHi.get<float4>(), parts);
+        bounds_final_kernel<<<1, 256, 0, s>>>(partLo, partHi, parts);
         PT_CUDA("centroid bounds", cudaGetLastError());
-        morton_kernel<<<grid_for(n, 256, 4096), 256, 0, s>>>(cent.get<float4>(), n, partLo.get<float4>(), partHi.get<float4>(),
-                                                             keys.get<uint32_t>(), values.get<uint32_t>());
+        morton_kernel<<<grid_for(n, 256, 4096), 256, 0, s>>>(cent, n, partLo, partHi, keys, values);
         PT_CUDA("morton codes", cudaGetLastError());
-        size_t tb = temp.bytes();
-        PT_CUDA("cub::DeviceRadixSort::SortPairs", cub::DeviceRadixSort::SortPairs(temp.get<void>(), tb, keys.get<uint32_t>(), keysSorted.get<uint32_t>(),
-                                                                                 values.get<uint32_t>(), sorted.get<uint32_t>(), static_cast<int>(n), 0, 30, s));
-        leaves_kernel<<<grid_for(n, 256, 4096), 256, 0, s>>>(sorted.get<uint32_t>(), n, triLo.get<float4>(), triHi.get<float4>(), lo.get<float4>(),
-                                                             hi.get<float4>(), child.get<uint2>(), clustersA.get<uint32_t>());
+        size_t tb = tempBytes;
+        PT_CUDA("cub::DeviceRadixSort::SortPairs", cub::DeviceRadixSort::SortPairs(temp, tb, keys, keysSorted, values, sorted,
+                                                                                 static_cast<int>(n), 0, 30, s));
+        leaves_kernel<<<grid_for(n, 256, 4096), 256, 0, s>>>(sorted, n, triLo, triHi, lo, hi, child, clustersA);
         PT_CUDA("leaves", cudaGetLastError());
 
-        // 3: clustering rounds; rounds[r] = first node index of round r (nodes of round r: [rounds[r], rounds[r + 1]))
-        std::vector<uint32_t> rounds{n};
-        uint32_t m = n, nodeBase = n;
-        uint32_t* cur = clustersA.get<uint32_t>();
-        uint32_t* nxt = clustersB.get<uint32_t>();
-        uint32_t totals[2] = {0, 0};
-        const uint32_t maxRounds = n + 8;  // every round merges at least the closest pair of its windows
-        while (m > 1)
+        // 3: clustering rounds
+        PlocState now{n, n, 0, 0};
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(state, &now, sizeof(now), cudaMemcpyHostToDevice, s));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(roundEnd, &n, 4, cudaMemcpyHostToDevice, s));
+        uint32_t* cur = clustersA;
+        uint32_t* nxt = clustersB;
+        while (now.clusters > kTailClusters)
         {
-            if (rounds.size() > maxRounds) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: clustering did not converge");
-            ploc_nearest_kernel<<<(m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(cur, m, lo.get<float4>(), hi.get<float4>(), nn.get<uint32_t>());
-            PT_CUDA("nearest clusters", cudaGetLastError());
-            ploc_flags_kernel<<<grid_for(m + 1, 256, 8192), 256, 0, s>>>(nn.get<uint32_t>(), m, merge.get<uint32_t>(), keep.get<uint32_t>());
-            PT_CUDA("cluster flags", cudaGetLastError());
-            tb = temp.bytes();
-            PT_CUDA("cub::DeviceScan::ExclusiveSum", cub::DeviceScan::ExclusiveSum(temp.get<void>(), tb, merge.get<uint32_t>(), mergePos.get<uint32_t>(),
-                                                                                  static_cast<int>(m + 1), s));
-            tb = temp.bytes();
-            PT_CUDA("cub::DeviceScan::ExclusiveSum", cub::DeviceScan::ExclusiveSum(temp.get<void>(), tb, keep.get<uint32_t>(), keepPos.get<uint32_t>(),
-                                                                                  static_cast<int>(m + 1), s));
-            ploc_merge_kernel<<<grid_for(m, 256, 8192), 256, 0, s>>>(cur, m, nn.get<uint32_t>(), merge.get<uint32_t>(), mergePos.get<uint32_t>(),
-                                                                     keep.get<uint32_t>(), keepPos.get<uint32_t>(), nodeBase, lo.get<float4>(),
-                                                                     hi.get<float4>(), child.get<uint2>(), nxt);
-            PT_CUDA("cluster merge", cudaGetLastError());
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&totals[0], mergePos.get<uint32_t>() + m, 4, cudaMemcpyDeviceToHost, s));
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&totals[1], keepPos.get<uint32_t>() + m, 4, cudaMemcpyDeviceToHost, s));
+            const uint32_t m = now.clusters;
+            for (int r = 0; r < kRoundsPerSync; r++)
+            {
+                ploc_nearest_kernel<<<(m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(cur, state, lo, hi, nn);
+                PT_CUDA("nearest clusters", cudaGetLastError());
+                ploc_flags_kernel<<<grid_for(m + 1, 256, 8192), 256, 0, s>>>(nn, state, m + 1, flags);
+                PT_CUDA("cluster flags", cudaGetLastError());
+                tb = tempBytes;
+                PT_CUDA("cub::DeviceScan::ExclusiveSum", cub::DeviceScan::ExclusiveSum(temp, tb, flags, ranks, static_cast<int>(m + 1), s));
+                ploc_merge_kernel<<<grid_for(m, 256, 8192), 256, 0, s>>>(cur, state, nn, flags, ranks, lo, hi, child, nxt);
+                PT_CUDA("cluster merge", cudaGetLastError());
+                ploc_advance_kernel<<<1, 1, 0, s>>>(state, ranks, roundEnd);
+                PT_CUDA("clustering round", cudaGetLastError());
+                std::swap(cur, nxt);
+            }
+            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&now, state, sizeof(now), cudaMemcpyDeviceToHost, s));
             PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(s));
-            if (totals[0] == 0 || totals[1] != m - totals[0])
-                return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a clustering round merged no pair");
-            nodeBase += totals[0];
-            m = totals[1];
-            rounds.push_back(nodeBase);
-            std::swap(cur, nxt);
+            if (now.stalled) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a clustering round merged no pair");
         }
-        if (nodeBase != nodes) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: clustering left the wrong number of nodes");
+        const uint32_t largeRounds = now.rounds;
+        ploc_tail_kernel<<<1, kTailClusters, 2 * kTailClusters * sizeof(float4), s>>>(cur, state, lo, hi, child, roundEnd);
+        PT_CUDA("last clustering rounds", cudaGetLastError());
+        std::vector<uint32_t> rounds(largeRounds + 1);
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(rounds.data(), roundEnd, rounds.size() * 4, cudaMemcpyDeviceToHost, s));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&now, state, sizeof(now), cudaMemcpyDeviceToHost, s));
+        PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(s));
+        if (now.stalled) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a clustering round merged no pair");
+        if (now.clusters != 1 || now.nodes != nodes) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: clustering left the wrong number of nodes");
         const uint32_t root = nodes - 1;
 
         // 4: collapse costs, one round at a time (children before parents)
-        collapse_leaf_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(n, lo.get<float4>(), hi.get<float4>(), cost.get<float>(), how.get<uint8_t>());
+        collapse_leaf_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(n, lo, hi, cost, how);
         PT_CUDA("collapse leaves", cudaGetLastError());
-        for (size_t r = 0; r + 1 < rounds.size(); r++)
+        for (uint32_t r = 0; r < largeRounds; r++)
         {
             const uint32_t a = rounds[r], b = rounds[r + 1];
-            collapse_node_kernel<<<grid_for(b - a, 128, 8192), 128, 0, s>>>(a, b, lo.get<float4>(), hi.get<float4>(), child.get<uint2>(), cost.get<float>(),
-                                                                            how.get<uint8_t>(), split.get<uint8_t>());
+            collapse_node_kernel<<<grid_for(b - a, 128, 8192), 128, 0, s>>>(a, b, lo, hi, child, cost, how, split);
+            PT_CUDA("collapse nodes", cudaGetLastError());
+        }
+        if (now.rounds > largeRounds)
+        {
+            collapse_tail_kernel<<<1, kTailClusters / 2, 0, s>>>(roundEnd, largeRounds, now.rounds, lo, hi, child, cost, how, split);
             PT_CUDA("collapse nodes", cudaGetLastError());
         }
 
         // 5: wide nodes level by level
         const uint32_t one = 1;
         const uint2 rootLevel = make_uint2(root, 0u);  // the root's header: record 0
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(levelA.get<uint2>(), &rootLevel, sizeof(rootLevel), cudaMemcpyHostToDevice, s));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(counter.get<uint32_t>(), &one, 4, cudaMemcpyHostToDevice, s));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(levelA, &rootLevel, sizeof(rootLevel), cudaMemcpyHostToDevice, s));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(counter, &one, 4, cudaMemcpyHostToDevice, s));
         uint32_t levelBase = 0, count = 1, depth = 0, allocated = 1;
-        uint2* level = levelA.get<uint2>();
-        uint2* nextLevel = levelB.get<uint2>();
+        uint2* level = levelA;
+        uint2* nextLevel = levelB;
         while (count > 0)
         {
             depth++;
             if (depth > kMaxStack) return Status::Err(GPT_ERR_CAPACITY, "BVH8 deeper than the traversal stack");
-            emit_level_kernel<<<grid_for(count, 128, 16384), 128, 0, s>>>(level, count, levelBase, levelBase + count, n, lo.get<float4>(), hi.get<float4>(),
-                                                                          child.get<uint2>(), how.get<uint8_t>(), split.get<uint8_t>(),
-                                                                          counter.get<uint32_t>(), nextLevel, wide.get<Record8>(),
-                                                                          headerRecord.get<uint32_t>(), nodeMasks.get<uint32_t>(),
-                                                                          leafRecord.get<uint32_t>(), n, errorFlags.get<uint32_t>());
+            emit_level_kernel<<<grid_for(count, 128, 16384), 128, 0, s>>>(level, count, levelBase, levelBase + count, n, lo, hi, child, how, split,
+                                                                          counter, nextLevel, wide, headerRecord, nodeMasks, leafRecord, n,
+                                                                          errorFlags);
             PT_CUDA("wide nodes", cudaGetLastError());
             uint32_t levelFlags = 0;
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&allocated, counter.get<uint32_t>(), 4, cudaMemcpyDeviceToHost, s));
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&levelFlags, errorFlags.get<uint32_t>(), 4, cudaMemcpyDeviceToHost, s));
+            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&allocated, counter, 4, cudaMemcpyDeviceToHost, s));
+            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&levelFlags, errorFlags, 4, cudaMemcpyDeviceToHost, s));
             PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(s));
             if (allocated > n) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: more wide nodes than the bound");
             if (levelFlags) break;  // reported below; the next level's list is incomplete
@@ -761,11 +923,11 @@ namespace pt
             count = allocated - levelBase;
             std::swap(level, nextLevel);
         }
-        uint32_t flags = 0;
-        PT_CUDA("cudaMemcpy", cudaMemcpy(&flags, errorFlags.get<void>(), 4, cudaMemcpyDeviceToHost));
-        if (flags & kBuildErrExponent) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "BVH build failed: BVH quantisation exponent overflow");
-        if (flags & kBuildErrCapacity) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide-node index beyond the node array");
-        if (flags) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide node's child list did not fit");
+        uint32_t failed = 0;
+        PT_CUDA("cudaMemcpy", cudaMemcpy(&failed, errorFlags, 4, cudaMemcpyDeviceToHost));
+        if (failed & kBuildErrExponent) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "BVH build failed: BVH quantisation exponent overflow");
+        if (failed & kBuildErrCapacity) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide-node index beyond the node array");
+        if (failed) return Status::Err(GPT_ERR_DEVICE_FAULT, "BVH build failed: a wide node's child list did not fit");
         if (allocated >= kMaxBlocks) return Status::Err(GPT_ERR_CAPACITY, "BVH8 has more than 2^24 nodes");
 
         // 6: the child blocks (empty slots stay zero)
@@ -774,17 +936,16 @@ namespace pt
         PT_TRY(out.blocks.allocate(blockBytes));
         PT_TRY(out.blockMasks.allocate(size_t(out.blockCount) * 4));
         PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(out.blocks.get<void>(), 0, blockBytes, s));
-        triangle_records_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(positions, models, sorted.get<uint32_t>(), leafRecord.get<uint32_t>(), n,
-                                                                       out.blocks.get<Record8>());
+        triangle_records_kernel<<<grid_for(n, 256, 8192), 256, 0, s>>>(positions, models, sorted, leafRecord, n, out.blocks.get<Record8>());
         PT_CUDA("triangle records", cudaGetLastError());
-        header_records_kernel<<<grid_for(allocated, 256, 8192), 256, 0, s>>>(wide.get<Record8>(), headerRecord.get<uint32_t>(), nodeMasks.get<uint32_t>(),
-                                                                             allocated, out.blocks.get<Record8>(), out.blockMasks.get<uint32_t>());
+        header_records_kernel<<<grid_for(allocated, 256, 8192), 256, 0, s>>>(wide, headerRecord, nodeMasks, allocated, out.blocks.get<Record8>(),
+                                                                             out.blockMasks.get<uint32_t>());
         PT_CUDA("header records", cudaGetLastError());
         PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(s));
         out.nodeCount = allocated;
         out.depth = depth;
         out.binaryNodes = nodes;
-        out.rounds = static_cast<uint32_t>(rounds.size() - 1);
+        out.rounds = now.rounds;
         return Status::Ok();
     }
 }

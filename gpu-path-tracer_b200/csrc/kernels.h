@@ -73,6 +73,10 @@ namespace pt
     cudaError_t launch_batch_trace(const SceneView& scene, uint32_t root, const float* rays, uint32_t n, uint32_t* cursor, uint32_t* triOut,
                                    float* uvtOut, uint8_t* occOut, int blocks, int threads, uint32_t* errorFlags, cudaStream_t stream,
                                    uint32_t bvhFormat = kBvh8Quantised);
+    // models[t] = model of triangle t's material (0 if its index is out of range); *mask: bit m = model m is present,
+    // bit kModelCount = an index is out of range.
+    cudaError_t launch_triangle_models(const uint32_t* materialIds, const MaterialDev* materials, uint32_t n, uint32_t materialCount, uint32_t* models,
+                                       uint32_t* mask, cudaStream_t stream);
     cudaError_t launch_shading_records(const float* positions, const float* normals, const float* tangents, const float* uvs,
                                        const uint32_t* materialIds, uint32_t n, float4* shading, cudaStream_t stream);
     cudaError_t launch_light_build(const float4* shading, const MaterialDev* materials, uint32_t n,

@@ -147,20 +147,38 @@ namespace pt
         NvtxRange rangeUpload("gpt scene upload");
         const auto tUpload = std::chrono::steady_clock::now();
         const uint32_t n = d.triangle_count;
-        std::vector<uint32_t> models(n);
-        bool present[kModelCount] = {};
         for (uint32_t m = 0; m < d.material_count; m++)
             if (d.materials[m].model >= kModelCount)
                 return Status::Err(GPT_ERR_INVALID_ARGUMENT, "Material has an unknown shading model");
-        for (uint32_t t = 0; t < n; t++)
-        {
-            const uint32_t mat = d.material_ids[t];
-            if (mat >= d.material_count) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "Triangle material index out of range");
-            models[t] = d.materials[mat].model;
-            present[models[t]] = true;
-        }
         auto scene = std::make_unique<SceneGpu>();
-        std::copy(present, present + kModelCount, scene->modelPresent);
+        // the upload's working arrays; the attributes are vertices as the caller has them
+        float *pos, *nrm, *tan, *uv;
+        uint32_t *mid, *modelsDev, *flags, *index, *lightCountDev, *modelMask;
+        double* scanScratch;
+        DeviceArena arena;
+        arena.add(pos, static_cast<size_t>(n) * 9);
+        arena.add(nrm, static_cast<size_t>(n) * 9);
+        arena.add(tan, static_cast<size_t>(n) * 12);
+        arena.add(uv, static_cast<size_t>(n) * 6);
+        arena.add(mid, n);
+        arena.add(modelsDev, n);
+        arena.add(flags, n);
+        arena.add(index, n);
+        arena.add(scanScratch, scan_scratch_elements(n));
+        arena.add(lightCountDev, 4);
+        arena.add(modelMask, 4);
+        PT_TRY(arena.allocate());
+        PT_TRY(scene->materials.allocate(static_cast<size_t>(d.material_count) * sizeof(MaterialDev)));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->materials.get<void>(), d.materials, static_cast<size_t>(d.material_count) * sizeof(MaterialDev), cudaMemcpyHostToDevice, stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(mid, d.material_ids, static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream));
+        // every triangle's shading model, the models present, and whether an index is out of range (a host loop
+        // over a million triangles took 3 ms)
+        PT_CUDA("triangle models", launch_triangle_models(mid, scene->materials.get<MaterialDev>(), n, d.material_count, modelsDev, modelMask, stream));
+        uint32_t mask = 0;
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&mask, modelMask, 4, cudaMemcpyDeviceToHost, stream));
+        PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream));
+        if (mask >> kModelCount) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "Triangle material index out of range");
+        for (uint32_t m = 0; m < kModelCount; m++) scene->modelPresent[m] = (mask >> m) & 1u;
         // image textures of the material slots
         if (d.texture_count > 0 && d.material_textures)
         {
@@ -191,9 +209,7 @@ namespace pt
                                                        cudaMemcpyHostToDevice, stream));
         }
         // Vertex positions go up first: the device BVH build and the shading records read them.
-        DeviceBuffer pos, nrm, tan, uv, mid;
-        PT_TRY(pos.allocate(static_cast<size_t>(n) * 9 * 4));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(pos.get<void>(), d.positions, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(pos, d.positions, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
         scene->triangleCount = n;
         scene->materialCount = d.material_count;
         scene->deviceBvh = deviceBvh;
@@ -203,11 +219,8 @@ namespace pt
         if (deviceBvh)
         {
             // BVH8 on the device (Morton order, clustering, collapse, quantisation); no binary BVH
-            DeviceBuffer modelsDev;
-            PT_TRY(modelsDev.allocate(static_cast<size_t>(n) * 4));
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(modelsDev.get<void>(), models.data(), static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream));
             DeviceBvh dev;
-            PT_TRY(BuildBvh8Device(pos.get<float>(), modelsDev.get<uint32_t>(), n, stream, dev));
+            PT_TRY(BuildBvh8Device(pos, modelsDev, n, stream, dev));
             scene->blocks.swap(dev.blocks);
             scene->blockMasks.swap(dev.blockMasks);
             scene->nodeCount = dev.nodeCount;
@@ -218,6 +231,8 @@ namespace pt
         else
         {
             // BVH8 on the host (binned SAH, collapse, quantisation).
+            std::vector<uint32_t> models(n);
+            for (uint32_t t = 0; t < n; t++) models[t] = d.materials[d.material_ids[t]].model;
             try
             {
                 bvh = BuildBvh8(d.positions, models.data(), n, static_cast<int>(std::max(1u, std::thread::hardware_concurrency())), withBinary);
@@ -239,7 +254,6 @@ namespace pt
         scene->bvhSeconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - tBvh).count();
         rangeBvh.end();
         PT_TRY(scene->shading.allocate(static_cast<size_t>(n) * 9 * sizeof(float4)));
-        PT_TRY(scene->materials.allocate(static_cast<size_t>(d.material_count) * sizeof(MaterialDev)));
         if (withBinary)
         {
             if (bvh.depth2 > kMaxStack) return Status::Err(GPT_ERR_CAPACITY, "Binary BVH deeper than the traversal stack");
@@ -249,49 +263,39 @@ namespace pt
             PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->nodes2.get<void>(), bvh.nodes2.data(), bvh.nodes2.size() * sizeof(Node2),
                                                        cudaMemcpyHostToDevice, stream));
         }
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(scene->materials.get<void>(), d.materials, static_cast<size_t>(d.material_count) * sizeof(MaterialDev), cudaMemcpyHostToDevice, stream));
         // Vertex attributes go up once; shading records, lights and the alias table are built on the device.
-        PT_TRY(nrm.allocate(static_cast<size_t>(n) * 9 * 4));
-        PT_TRY(tan.allocate(static_cast<size_t>(n) * 12 * 4));
-        PT_TRY(uv.allocate(static_cast<size_t>(n) * 6 * 4));
-        PT_TRY(mid.allocate(static_cast<size_t>(n) * 4));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(nrm.get<void>(), d.normals, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(tan.get<void>(), d.tangents, static_cast<size_t>(n) * 48, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(uv.get<void>(), d.uvs, static_cast<size_t>(n) * 24, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(mid.get<void>(), d.material_ids, static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("shading records", launch_shading_records(pos.get<float>(), nrm.get<float>(), tan.get<float>(), uv.get<float>(), mid.get<uint32_t>(), n,
-                                                          scene->shading.get<float4>(), stream));
-        DeviceBuffer flags, index, scanScratch, lightCountDev;
-        PT_TRY(flags.allocate(static_cast<size_t>(n) * 4));
-        PT_TRY(index.allocate(static_cast<size_t>(n) * 4));
-        PT_TRY(scanScratch.allocate(scan_scratch_elements(n) * 8));
-        PT_TRY(lightCountDev.allocate(16));
-        PT_CUDA("light build", launch_light_build(scene->shading.get<float4>(), scene->materials.get<MaterialDev>(), n,
-                                                  flags.get<uint32_t>(), index.get<uint32_t>(), scanScratch.get<uint32_t>(), lightCountDev.get<uint32_t>(), stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(nrm, d.normals, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(tan, d.tangents, static_cast<size_t>(n) * 48, cudaMemcpyHostToDevice, stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(uv, d.uvs, static_cast<size_t>(n) * 24, cudaMemcpyHostToDevice, stream));
+        PT_CUDA("shading records", launch_shading_records(pos, nrm, tan, uv, mid, n, scene->shading.get<float4>(), stream));
+        PT_CUDA("light build", launch_light_build(scene->shading.get<float4>(), scene->materials.get<MaterialDev>(), n, flags, index,
+                                                  reinterpret_cast<uint32_t*>(scanScratch), lightCountDev, stream));
         uint32_t lightCount = 0;
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&lightCount, lightCountDev.get<void>(), 4, cudaMemcpyDeviceToHost, stream));
+        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&lightCount, lightCountDev, 4, cudaMemcpyDeviceToHost, stream));
         PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream));
         scene->lightCount = lightCount;
         if (lightCount > 0)
         {
-            DeviceBuffer weights, powerWeights, powerScratch, prefix, stackIndex, stackValue;
+            double *weights, *powerWeights, *prefix;
+            uint32_t* stackIndex;
+            float* stackValue;
+            char* powerScratch;
+            DeviceArena lightArena;
+            lightArena.add(weights, lightCount);
+            lightArena.add(powerWeights, lightCount);
+            lightArena.add(prefix, lightCount);
+            lightArena.add(stackIndex, static_cast<size_t>(lightCount) * 2);
+            lightArena.add(stackValue, static_cast<size_t>(lightCount) * 2);
+            lightArena.add(powerScratch, alias_power_scratch_bytes(lightCount));
+            PT_TRY(lightArena.allocate());
             PT_TRY(scene->lights.allocate(static_cast<size_t>(lightCount) * 7 * sizeof(float4)));
             PT_TRY(scene->bins.allocate(static_cast<size_t>(lightCount) * sizeof(uint4)));
             PT_TRY(scene->binsPower.allocate(static_cast<size_t>(lightCount) * sizeof(uint4)));
-            PT_TRY(weights.allocate(static_cast<size_t>(lightCount) * 8));
-            PT_TRY(powerWeights.allocate(static_cast<size_t>(lightCount) * 8));
-            PT_TRY(powerScratch.allocate(alias_power_scratch_bytes(lightCount)));
-            PT_TRY(prefix.allocate(static_cast<size_t>(lightCount) * 8));
-            PT_TRY(stackIndex.allocate(static_cast<size_t>(lightCount) * 8));
-            PT_TRY(stackValue.allocate(static_cast<size_t>(lightCount) * 8));
             const MaterialTextures* tex = scene->textures.empty() ? nullptr : scene->materialTextures.get<MaterialTextures>();
-            PT_CUDA("light records", launch_light_records(pos.get<float>(), scene->shading.get<float4>(), scene->materials.get<MaterialDev>(), tex,
-                                                          n, flags.get<uint32_t>(), index.get<uint32_t>(), scene->lights.get<float4>(),
-                                                          weights.get<double>(), powerWeights.get<double>(), stream));
-            PT_CUDA("alias table", launch_alias_build(weights.get<double>(), lightCount, prefix.get<double>(), scanScratch.get<double>(),
-                                                      scene->bins.get<uint4>(), stackIndex.get<uint32_t>(), stackValue.get<float>(), stream));
-            PT_CUDA("power alias table", launch_alias_build_power(powerWeights.get<double>(), weights.get<double>(), lightCount,
-                                                                  powerScratch.get<void>(), scene->binsPower.get<uint4>(), stream));
+            PT_CUDA("light records", launch_light_records(pos, scene->shading.get<float4>(), scene->materials.get<MaterialDev>(), tex, n, flags, index,
+                                                          scene->lights.get<float4>(), weights, powerWeights, stream));
+            PT_CUDA("alias table", launch_alias_build(weights, lightCount, prefix, scanScratch, scene->bins.get<uint4>(), stackIndex, stackValue, stream));
+            PT_CUDA("power alias table", launch_alias_build_power(powerWeights, weights, lightCount, powerScratch, scene->binsPower.get<uint4>(), stream));
             PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream));
         }
         const SceneEntry entry{0u, 0u, lightCount, 0u};

@@ -108,6 +108,35 @@ namespace pt
         size_t bytes_ = 0;
     };
 
+    // Several device arrays in one allocation: add() every array, then allocate(). A cudaMalloc and a cudaFree
+    // cost 0.1 to 0.3 ms each, whatever their size, and the free waits for the device.
+    class DeviceArena
+    {
+    public:
+        template <typename T>
+        void add(T*& array, size_t count)
+        {
+            parts_.push_back({reinterpret_cast<void**>(&array), bytes_});
+            bytes_ += (count * sizeof(T) + 255) / 256 * 256;
+        }
+        Status allocate()
+        {
+            PT_TRY(buffer_.allocate(bytes_));
+            for (const Part& p : parts_) *p.array = buffer_.get<char>() + p.offset;
+            return Status::Ok();
+        }
+
+    private:
+        struct Part
+        {
+            void** array;
+            size_t offset;
+        };
+        DeviceBuffer buffer_;
+        std::vector<Part> parts_;
+        size_t bytes_ = 0;
+    };
+
     // An image texture with the reference's descriptors (Texture.cpp:65-189).
     struct TextureObject
     {

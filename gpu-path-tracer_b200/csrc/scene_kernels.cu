@@ -511,6 +511,31 @@ namespace pt
         }
     }
 
+    __global__ void triangle_models_kernel(const uint32_t* materialIds, const MaterialDev* materials, uint32_t n, uint32_t materialCount,
+                                           uint32_t* models, uint32_t* mask)
+    {
+        uint32_t seen = 0;
+        for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+        {
+            const uint32_t mat = materialIds[t];
+            const uint32_t model = mat < materialCount ? materials[mat].model : 0u;
+            models[t] = model;
+            seen |= 1u << (mat < materialCount ? model : kModelCount);
+        }
+        seen = __reduce_or_sync(0xFFFFFFFFu, seen);
+        if (scan_lane_id() == 0 && seen != 0) atomicOr(mask, seen);
+    }
+
+    cudaError_t launch_triangle_models(const uint32_t* materialIds, const MaterialDev* materials, uint32_t n, uint32_t materialCount, uint32_t* models,
+                                       uint32_t* mask, cudaStream_t s)
+    {
+        cudaError_t e = cudaMemsetAsync(mask, 0, 4, s);
+        if (e != cudaSuccess) return e;
+        const uint32_t blocks = (n + 255) / 256 < 2048 ? (n + 255) / 256 : 2048;
+        triangle_models_kernel<<<blocks ? blocks : 1, 256, 0, s>>>(materialIds, materials, n, materialCount, models, mask);
+        return cudaGetLastError();
+    }
+
     cudaError_t launch_shading_records(const float* positions, const float* normals, const float* tangents, const float* uvs,
                                        const uint32_t* materialIds, uint32_t n, float4* shading, cudaStream_t s)
     {

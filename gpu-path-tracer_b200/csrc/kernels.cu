@@ -878,12 +878,16 @@ namespace pt
                 wf.regenBits[i] = 0u;
     }
 
-    // Regeneration from the finished-slot bitmap: each warp takes a tile of 32 bitmap words (1,024
-    // slots), reserves new samples for the tile's finished paths with one atomic, and walks the words in
+    // Regeneration from the finished-slot bitmap: each warp takes a tile of kRegenTile bitmap words, reserves new samples for the tile's finished paths with one atomic, and walks the words in
     // slot order, so the slot records of finished and new paths are read and written in address order
     // (the queue holds them in the order paths finished, i.e. scattered). The set of new samples, their
     // ray-queue positions and every sample's result are those of the queue-driven regeneration; only
     // which slot a new sample lands in differs.
+    // Bitmap words of a warp's tile. A pool of 1,048,576 slots is 4,096 tiles of 8 words, but only 1,024 tiles of
+    // 32, each walked by one warp of an otherwise empty GPU: the Cornell box frame's regeneration took 0.43
+    // instead of 0.23 ms, the 640x360 preview's 0.042 instead of 0.022 ms (16 words 0.29 and 0.028, 4 words 0.24
+    // and 0.020). With 16,777,216 slots 8, 16 and 32 words measure the same 5.0 ms, 4 words 5.2 ms.
+    constexpr uint32_t kRegenTile = 8;
     constexpr uint32_t kRegenGroup = 4;  // bitmap words whose finished slots are loaded together
 
     __global__ void regen_bits_kernel(Wavefront wf, const JobView* jobPtr)
@@ -898,14 +902,14 @@ namespace pt
         const uint32_t base = ctr->rayCount[nxt].v;
         float* out = jobPtr->sampleRadiance;
         const uint32_t words = (wf.capacity + 31u) >> 5;
-        const uint32_t tiles = (words + 31u) >> 5;
+        const uint32_t tiles = (words + kRegenTile - 1u) / kRegenTile;
         const uint32_t lane = lane_id();
         const uint32_t lanesBelow = (1u << lane) - 1u;
         const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
         for (uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < tiles; tile += warps)
         {
-            const uint32_t wi = tile * 32u + lane;
-            const uint32_t bits = wi < words ? wf.regenBits[wi] : 0u;
+            const uint32_t wi = tile * kRegenTile + lane;
+            const uint32_t bits = lane < kRegenTile && wi < words ? wf.regenBits[wi] : 0u;
             if (bits) wf.regenBits[wi] = 0u;
             const uint32_t count = static_cast<uint32_t>(__popc(bits));
             uint32_t incl = count;
@@ -921,7 +925,7 @@ namespace pt
             first = __shfl_sync(0xFFFFFFFFu, first, 0);
             const uint32_t excl = incl - count;
             // words in groups of kRegenGroup: the finished slots' loads of a group are in flight together
-            for (uint32_t jb = 0; jb < 32; jb += kRegenGroup)
+            for (uint32_t jb = 0; jb < kRegenTile; jb += kRegenGroup)
             {
                 uint32_t w[kRegenGroup], offset[kRegenGroup], sample[kRegenGroup];
                 float4 L[kRegenGroup];
@@ -934,7 +938,7 @@ namespace pt
                     sample[q] = 0;
                     if ((w[q] >> lane) & 1u)
                     {
-                        const uint32_t slot = (tile * 32u + jb + q) * 32u + lane;
+                        const uint32_t slot = (tile * kRegenTile + jb + q) * 32u + lane;
                         L[q] = wf.slotL[slot];
                         sample[q] = wf.slotSample[slot];
                     }
@@ -943,7 +947,7 @@ namespace pt
                 for (uint32_t q = 0; q < kRegenGroup; q++)
                 {
                     if (!((w[q] >> lane) & 1u)) continue;
-                    const uint32_t slot = (tile * 32u + jb + q) * 32u + lane;
+                    const uint32_t slot = (tile * kRegenTile + jb + q) * 32u + lane;
                     float* dst = out + static_cast<size_t>(sample[q]) * 3;
                     dst[0] = L[q].x;
                     dst[1] = L[q].y;
@@ -1943,7 +1947,7 @@ namespace pt
         const uint32_t nxt = ctr->cur ^ 1u;
         const uint32_t base = ctr->rayCount[nxt].v;
         const uint32_t words = (wf.capacity + 31u) >> 5;
-        const uint32_t tiles = (words + 31u) >> 5;
+        const uint32_t tiles = (words + kRegenTile - 1u) / kRegenTile;
         const uint32_t lane = lane_id();
         const uint32_t lanesBelow = (1u << lane) - 1u;
         const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -1962,8 +1966,8 @@ namespace pt
         const LaunchSegment* segments = shared ? localSegments : ev.segments;
         for (uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < tiles; tile += warps)
         {
-            const uint32_t wi = tile * 32u + lane;
-            const uint32_t bits = wi < words ? wf.regenBits[wi] : 0u;
+            const uint32_t wi = tile * kRegenTile + lane;
+            const uint32_t bits = lane < kRegenTile && wi < words ? wf.regenBits[wi] : 0u;
             if (bits) wf.regenBits[wi] = 0u;
             const uint32_t count = static_cast<uint32_t>(__popc(bits));
             uint32_t incl = count;
@@ -1979,7 +1983,7 @@ namespace pt
             first = __shfl_sync(0xFFFFFFFFu, first, 0);
             const uint32_t excl = incl - count;
             // words in groups of kRegenGroup: the finished slots' loads of a group are in flight together
-            for (uint32_t jb = 0; jb < 32; jb += kRegenGroup)
+            for (uint32_t jb = 0; jb < kRegenTile; jb += kRegenGroup)
             {
                 uint32_t w[kRegenGroup], offset[kRegenGroup], meta[kRegenGroup], sample[kRegenGroup];
                 float4 L[kRegenGroup];
@@ -1993,7 +1997,7 @@ namespace pt
                     sample[q] = 0;
                     if ((w[q] >> lane) & 1u)
                     {
-                        const uint32_t slot = (tile * 32u + jb + q) * 32u + lane;
+                        const uint32_t slot = (tile * kRegenTile + jb + q) * 32u + lane;
                         meta[q] = __float_as_uint(wf.slotT[slot].w);
                         sample[q] = wf.slotSample[slot];
                         L[q] = wf.slotL[slot];
@@ -2003,7 +2007,7 @@ namespace pt
                 for (uint32_t q = 0; q < kRegenGroup; q++)
                 {
                     if (!((w[q] >> lane) & 1u)) continue;
-                    const uint32_t slot = (tile * 32u + jb + q) * 32u + lane;
+                    const uint32_t slot = (tile * kRegenTile + jb + q) * 32u + lane;
                     engine_retire_path(ev, meta[q], sample[q], L[q], passKey, passCount);
                     const uint32_t k = first + offset[q] + static_cast<uint32_t>(__popc(w[q] & lanesBelow));
                     if (k < launch) engine_start_launch(wf, ev, segments, k, slot, segmentCount, nxt, base);

@@ -341,7 +341,7 @@ namespace pt
             if (!pending_.empty() || !active_.empty()) return Status::Err(GPT_ERR_STATE, "Scenes are added while no job is queued or running");
             PT_CUDA("cudaSetDevice", cudaSetDevice(device_));
             std::unique_ptr<SceneGpu> scene;
-            PT_TRY(BuildScene(d, stream_, scene, false, cfg_.bvh_build == GPT_BVH_BUILD_DEVICE));
+            PT_TRY(BuildScene(d, stream_, upload_, scene, false, cfg_.bvh_build == GPT_BVH_BUILD_DEVICE));
             PT_TRY(AppendScene(pack_, *scene, stream_));
             releaseGraph();
             id = static_cast<uint32_t>(pack_.entry.size() - 1);
@@ -1037,6 +1037,7 @@ namespace pt
         DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regenBits_, slotT_, slotL_, slotSample_, freeList_;
         DeviceBuffer counters_, ctl_, jobs_, order_, segments_;
         ScenePack pack_;
+        PinnedUpload upload_;
         Arena arena_;
         cudaGraph_t graph_ = nullptr;
         cudaGraphExec_t graphExec_ = nullptr;

@@ -139,7 +139,7 @@ namespace pt
 
     // Scene upload of Renderer::InitializeSceneBuffers (Renderer.cpp:292-306): validation, image textures,
     // BVH8 (host or device), shading records, light list and alias table (device).
-    Status BuildScene(const gpt_scene_desc& d, cudaStream_t stream, std::unique_ptr<SceneGpu>& out, bool withBinary, bool deviceBvh)
+    Status BuildScene(const gpt_scene_desc& d, cudaStream_t stream, PinnedUpload& upload, std::unique_ptr<SceneGpu>& out, bool withBinary, bool deviceBvh)
     {
         if (d.triangle_count == 0 || !d.positions || !d.normals || !d.tangents || !d.uvs || !d.material_ids || !d.materials ||
             d.material_count == 0)
@@ -209,7 +209,12 @@ namespace pt
                                                        cudaMemcpyHostToDevice, stream));
         }
         // Vertex positions go up first: the device BVH build and the shading records read them.
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(pos, d.positions, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
+        PinnedUpload::Job job;
+        PT_TRY(upload.start(job, {{pos, d.positions, static_cast<size_t>(n) * 36}}, stream));
+        PT_TRY(job.wait());
+        // the attributes, wanted by the shading records behind the BVH build
+        PT_TRY(upload.start(job, {{nrm, d.normals, static_cast<size_t>(n) * 36}, {tan, d.tangents, static_cast<size_t>(n) * 48}, {uv, d.uvs, static_cast<size_t>(n) * 24}},
+                            stream));
         scene->triangleCount = n;
         scene->materialCount = d.material_count;
         scene->deviceBvh = deviceBvh;
@@ -264,9 +269,7 @@ namespace pt
                                                        cudaMemcpyHostToDevice, stream));
         }
         // Vertex attributes go up once; shading records, lights and the alias table are built on the device.
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(nrm, d.normals, static_cast<size_t>(n) * 36, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(tan, d.tangents, static_cast<size_t>(n) * 48, cudaMemcpyHostToDevice, stream));
-        PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(uv, d.uvs, static_cast<size_t>(n) * 24, cudaMemcpyHostToDevice, stream));
+        PT_TRY(job.wait());
         PT_CUDA("shading records", launch_shading_records(pos, nrm, tan, uv, mid, n, scene->shading.get<float4>(), stream));
         PT_CUDA("light build", launch_light_build(scene->shading.get<float4>(), scene->materials.get<MaterialDev>(), n, flags, index,
                                                   reinterpret_cast<uint32_t*>(scanScratch), lightCountDev, stream));
@@ -433,7 +436,7 @@ namespace pt
             if (rendering_.load()) return Status::Err(GPT_ERR_STATE, "Cannot upload a scene while rendering");
             PT_CUDA("cudaSetDevice", cudaSetDevice(device_));
             std::unique_ptr<SceneGpu> scene;
-            PT_TRY(BuildScene(d, stream_, scene, true, bvhBuild_ == GPT_BVH_BUILD_DEVICE));
+            PT_TRY(BuildScene(d, stream_, upload_, scene, true, bvhBuild_ == GPT_BVH_BUILD_DEVICE));
             releaseGraph();
             scene->version = ++sceneVersion_;
             scene_ = std::move(scene);
@@ -994,6 +997,7 @@ namespace pt
         JobView hostJob_{};
         Counters hostCounters_{};
         std::unique_ptr<SceneGpu> scene_;
+        PinnedUpload upload_;
         uint64_t sceneVersion_ = 0;
         uint32_t width_ = 0, height_ = 0;
         std::vector<uint32_t> hostFrame_;

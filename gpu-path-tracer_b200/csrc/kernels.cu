@@ -578,6 +578,151 @@ namespace pt
     }
 
 
+    // Few rays: a warp per ray. With a lane per ray, 10,000 rays are 312 warps, which cannot hide their loads,
+    // and the launch lasts as long as its longest ray: the last iterations of every frame, with some rays left,
+    // took about 35 us per launch. Here up to 4 nodes off the top of the ray's stack are visited at once, each by
+    // 8 lanes that test a child each, and the triangles of all their leaves at once; nodes behind the closest hit
+    // are dropped. 640x360 preview frame of spheres-200k: 0.80 -> 0.54 ms on the device; textured room 333x217x9:
+    // 0.72 -> 0.64 ms; large frames 0.4 ms. Up to kFewRays rays per warp of the grid: 2 took the preview 0.60 ms,
+    // 8 the same as 4, 16 slowed the Cornell box frame from 3.38 to 3.48 ms. (8 lanes per ray and one node at a
+    // time, for 32 to 64 rays per warp, was slower than a lane per ray: preview 0.64 to 0.69 ms.)
+    constexpr uint32_t kFewRays = 4;
+    constexpr int kFewNodes = 4;
+
+    // stack: 32 * STACK words of the warp: 16 * STACK records and as many entry distances. From at most
+    // 9 * STACK - 32 records on the stack several nodes are taken, which leaves at most 9 * STACK - 4; one node at
+    // a time then adds at most 7 per level of its subtree (trees are at most STACK levels deep).
+    template <int STACK, bool ANY, class Work>
+    __device__ __forceinline__ void trace_few(const Work& work, uint32_t n, uint32_t* stack, uint32_t& visits, uint32_t& tests)
+    {
+        constexpr uint32_t kCapacity = 16u * STACK;
+        constexpr int kSeveral = 9 * STACK - 32;
+        float* entry = reinterpret_cast<float*>(stack + kCapacity);
+        const uint32_t lane = lane_id(), group = lane >> 3, child = lane & 7u;
+        const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+        for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps)
+        {
+            float3 o, d;
+            float tmin, tmax;
+            uint32_t tag;
+            work.load(i, o, d, tmin, tmax, tag);
+            const RayPre ray = make_ray(o, d, tmin);
+            const uint32_t oct = ANY ? ray.oct ^ 7u : ray.oct;
+            HitRecord best{tmax, kInvalid, 0.0f, 0.0f, 0u};
+            bool occluded = false;
+            int sp = 1;
+            if (lane == 0)
+            {
+                stack[0] = work.root(tag) * kBlockRecords;
+                entry[0] = tmin;
+            }
+            __syncwarp();
+            while (sp > 0)
+            {
+                const int take = sp <= kSeveral ? (sp < kFewNodes ? sp : kFewNodes) : 1;
+                sp -= take;
+                uint32_t record = 0;
+                bool live = static_cast<int>(group) < take;
+                if (live)
+                {
+                    const int at = sp + take - 1 - static_cast<int>(group);
+                    record = stack[at];
+                    live = !(entry[at] > best.t);
+                }
+                bool hit = false, inner = false;
+                float tn = 0.0f;
+                if (live)
+                {
+                    const uint4* nw = work.sc.records[record].w;
+                    uint4 w0, w1, w2, w3;
+                    ldg8(nw, w0, w1);
+                    ldg8(nw + 2, w2, w3);
+                    hit = intersect_child(w0, w1, w2, w3, ray, child, tmin, best.t, tn);
+                    inner = (w0.x >> child) & 1u;
+                    record = (w0.w >> 8) * kBlockRecords + child;
+                    if (child == 0) visits++;
+                }
+                if (__ballot_sync(0xFFFFFFFFu, hit && !inner))
+                {
+                    bool found = false;
+                    float t = 0.0f, u = 0.0f, v = 0.0f;
+                    uint32_t tri = kInvalid, model = 0;
+                    if (hit && !inner)
+                    {
+                        uint32_t next = record;
+                        do
+                        {
+                            tests++;
+                            const uint4* tp = work.sc.records[next].w;
+                            uint4 ua, ub;
+                            ldg8(tp, ua, ub);
+                            const float4 a = make_float4(__uint_as_float(ua.x), __uint_as_float(ua.y), __uint_as_float(ua.z), 0.0f);
+                            const float4 b = make_float4(__uint_as_float(ub.x), __uint_as_float(ub.y), __uint_as_float(ub.z), 0.0f);
+                            const float4 e = ldg4(reinterpret_cast<const float4*>(tp + 2));
+                            next = __float_as_uint(e.w);
+                            float ht, hu, hv;
+                            if (intersect_triangle(a, b, e, o, d, ht, hu, hv) && ht >= tmin && (ANY ? ht < tmax : ht <= best.t) &&
+                                (!found || ht < t || (ht == t && ua.w < tri)))
+                            {
+                                found = true;
+                                t = ht;
+                                u = hu;
+                                v = hv;
+                                tri = ua.w;
+                                model = ub.w;
+                            }
+                        } while (next != 0u);
+                    }
+                    if (ANY)
+                    {
+                        if (__ballot_sync(0xFFFFFFFFu, found))
+                        {
+                            occluded = true;
+                            break;
+                        }
+                    }
+                    else
+                    {
+                        // the nearest of the lanes' hits, the smallest triangle index among equals
+                        const uint32_t bits = __float_as_uint(t + 0.0f);
+                        const uint32_t key = found ? bits ^ (static_cast<uint32_t>(static_cast<int32_t>(bits) >> 31) | 0x80000000u) : 0xFFFFFFFFu;
+                        const uint32_t least = __reduce_min_sync(0xFFFFFFFFu, key);
+                        if (least != 0xFFFFFFFFu)
+                        {
+                            const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, key == least ? tri : kInvalid);
+                            const int owner = __ffs(__ballot_sync(0xFFFFFFFFu, key == least && tri == first)) - 1;
+                            t = __shfl_sync(0xFFFFFFFFu, t, owner);
+                            u = __shfl_sync(0xFFFFFFFFu, u, owner);
+                            v = __shfl_sync(0xFFFFFFFFu, v, owner);
+                            model = __shfl_sync(0xFFFFFFFFu, model, owner);
+                            if (t < best.t || (best.tri != kInvalid && first < best.tri)) best = HitRecord{t, first, u, v, model};
+                        }
+                    }
+                }
+                // inner children in front of the closest hit: nearest nodes' children, and of a node the first in
+                // visiting order, on top
+                const bool push = hit && inner && !(tn > best.t);
+                uint32_t pushed = __ballot_sync(0xFFFFFFFFu, push);
+                const int count = __popc(pushed);
+                if (oct & 1u) pushed = ((pushed & 0x55555555u) << 1) | ((pushed >> 1) & 0x55555555u);
+                if (oct & 2u) pushed = ((pushed & 0x33333333u) << 2) | ((pushed >> 2) & 0x33333333u);
+                if (oct & 4u) pushed = ((pushed & 0x0F0F0F0Fu) << 4) | ((pushed >> 4) & 0x0F0F0F0Fu);
+                const uint32_t place = (group << 3) | (child ^ oct);
+                __syncwarp();
+                if (push)
+                {
+                    const int at = sp + __popc(pushed & ~((2u << place) - 1u));
+                    stack[at] = record;
+                    entry[at] = tn;
+                }
+                sp += count;
+                __syncwarp();
+            }
+            if (lane == 0) work.finish(i, tag, best, occluded, o, d);
+            __syncwarp();
+        }
+    }
+
     // The same for the BVH8, with the warp's lanes in step: each step visits a few nodes per lane, then tests
     // one triangle per lane if enough lanes hold leaves (kLeafShare), and goes on testing while more than
     // half of the busy lanes do. A node visit rarely enters leaves in more than a few lanes (0.34 tests per
@@ -623,7 +768,11 @@ namespace pt
         int waiting = 0;
         bool active = false;     // a ray in flight (finished or not)
         bool exhausted = false;
-        for (;;)
+        // (a caller's smaller stack is a test of the lane path's bound)
+        const bool few = work.stackCap == 0 && n <= kFewRays * ((gridDim.x * blockDim.x) >> 5);
+        if (few)
+            trace_few<STACK, ANY>(work, n, reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + (threadIdx.x >> 5) * 32u * STACK, visits, tests);
+        else for (;;)
         {
             const bool over = st.sp == 0 && leaves == 0;
             const unsigned idle = __ballot_sync(0xFFFFFFFFu, over);

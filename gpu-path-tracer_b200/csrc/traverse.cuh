@@ -124,26 +124,37 @@ namespace pt
         missed = __funnelshift_l(__float_as_uint(tf - tn), missed, 1);
     }
 
+    // A node's origin relative to the ray's, and its box scales.
+    // unit = 2^(u - 127) is 2^-8 of the origin's grid (the low byte of a word is masked, so it holds
+    // 256 q); the shift leaves a bit of q in the sign, which fabsf drops. Scales are unit * 2^(e + 1).
+    // Powers of two: origin and scale are exact, and d rounds once.
+    struct NodeFrame
+    {
+        float3 d, s;
+    };
+    __device__ __forceinline__ NodeFrame node_frame(uint4 w0, const RayPre& r)
+    {
+        const float unit = fabsf(as_float(w0.y << 23));
+        NodeFrame f;
+        f.s = make_float3(as_float(((w0.z << 23) & 0x0F800000u) | 0x40000000u) * unit, as_float(((w0.w << 23) & 0x0F800000u) | 0x40000000u) * unit,
+                          as_float(((w0.z << 18) & 0x03800000u) | ((w0.w << 21) & 0x0C000000u) | 0x40000000u) * unit);
+        f.d = make_float3(__fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.x & ~0xFFu)), unit, -r.o.x),
+                          __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.y & ~0xFFu)), unit, -r.o.y),
+                          __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.z & ~0xFFu)), unit, -r.o.z));
+        return f;
+    }
+
     // Slab test of the 8 quantised children against [tmin, tmax], conservative for every child box (a box the
     // exact arithmetic would hit is never culled). Returns the hit mask in slot order. Empty slots hold inverted
     // boxes and are almost always culled; one that passes is a record of zeros, which no ray hits.
     template <bool FIXED>
     __device__ __forceinline__ uint32_t intersect_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, float tmin, float tmax)
     {
-        // unit = 2^(u - 127) is 2^-8 of the origin's grid (the low byte of a word is masked, so it holds
-        // 256 q); the shift leaves a bit of q in the sign, which fabsf drops. Scales are unit * 2^(e + 1).
-        // Powers of two: origin and scale are exact, and dx, dy, dz round once.
-        const float unit = fabsf(as_float(w0.y << 23));
-        const float sx = as_float(((w0.z << 23) & 0x0F800000u) | 0x40000000u) * (unit * 32768.0f);
-        const float sy = as_float(((w0.w << 23) & 0x0F800000u) | 0x40000000u) * unit;
-        const float sz = as_float(((w0.z << 18) & 0x03800000u) | ((w0.w << 21) & 0x0C000000u) | 0x40000000u) * unit;
-        const float dx = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.x & ~0xFFu)), unit, -r.o.x);
-        const float dy = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.y & ~0xFFu)), unit, -r.o.y);
-        const float dz = __fmaf_rn(static_cast<float>(static_cast<int32_t>(w0.z & ~0xFFu)), unit, -r.o.z);
+        const NodeFrame f = node_frame(w0, r);
         // qlo.x = w1.xy, qlo.y = w1.zw, qlo.z = w2.xy, qhi.x = w2.zw, qhi.y = w3.xy, qhi.z = w3.zw
-        const SlabAxis x = slab_axis<true>(dx, sx, r.invd.x, w1.x, w1.y, w2.z, w2.w);
-        const SlabAxis y = slab_axis<false>(dy, sy, r.invd.y, w1.z, w1.w, w3.x, w3.y);
-        const SlabAxis z = slab_axis<false>(dz, sz, r.invd.z, w2.x, w2.y, w3.z, w3.w);
+        const SlabAxis x = slab_axis<true>(f.d.x, f.s.x * 32768.0f, r.invd.x, w1.x, w1.y, w2.z, w2.w);
+        const SlabAxis y = slab_axis<false>(f.d.y, f.s.y, r.invd.y, w1.z, w1.w, w3.x, w3.y);
+        const SlabAxis z = slab_axis<false>(f.d.z, f.s.z, r.invd.z, w2.x, w2.y, w3.z, w3.w);
         uint32_t missed = 0;
         slab_child<7, FIXED>(x, y, z, tmin, tmax, missed);
         slab_child<6, FIXED>(x, y, z, tmin, tmax, missed);
@@ -154,6 +165,22 @@ namespace pt
         slab_child<1, FIXED>(x, y, z, tmin, tmax, missed);
         slab_child<0, FIXED>(x, y, z, tmin, tmax, missed);
         return ~missed & 0xFFu;
+    }
+
+    // The same test for child c alone, with its entry distance.
+    __device__ __forceinline__ bool intersect_child(uint4 w0, uint4 w1, uint4 w2, uint4 w3, const RayPre& r, uint32_t c, float tmin, float tmax, float& tn)
+    {
+        const NodeFrame f = node_frame(w0, r);
+        const SlabAxis x = slab_axis<false>(f.d.x, f.s.x, r.invd.x, w1.x, w1.y, w2.z, w2.w);
+        const SlabAxis y = slab_axis<false>(f.d.y, f.s.y, r.invd.y, w1.z, w1.w, w3.x, w3.y);
+        const SlabAxis z = slab_axis<false>(f.d.z, f.s.z, r.invd.z, w2.x, w2.y, w3.z, w3.w);
+        const uint32_t shift = (c & 3u) * 8u;
+        const bool high = c >= 4u;
+        const auto plane = [&](uint32_t lo, uint32_t hi, float a, float b)
+        { return __fmaf_rn(static_cast<float>(((high ? hi : lo) >> shift) & 0xFFu), a, b); };
+        tn = fmaxf(max3f(plane(x.nearLo, x.nearHi, x.a, x.near), plane(y.nearLo, y.nearHi, y.a, y.near), plane(z.nearLo, z.nearHi, z.a, z.near)), tmin);
+        const float tf = fminf(min3f(plane(x.farLo, x.farHi, x.a, x.far), plane(y.farLo, y.farHi, y.a, y.far), plane(z.farLo, z.farHi, z.a, z.far)), tmax);
+        return !(tn > tf);
     }
 
     // Moller-Trumbore with the reference's determinant cull and inclusive edges

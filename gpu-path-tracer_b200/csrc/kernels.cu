@@ -52,10 +52,15 @@ namespace pt
         return t;
     }
 
-    // Phase timing: thread 0 of every block stamps its start (min) and its end (max).
+    // Phase timing: thread 0 of block 0 stamps the start (the least of the shading kernels'), thread 0 of every
+    // block that had work its end (the largest). Blocks without work stamp nothing and leave at once: a kernel
+    // does not end before its atomics have, which queue up on one address, and a traversal launch's 1,332 blocks
+    // with two stamps each and two sums per warp made 13,000 of them for the few rays of a frame's last
+    // iterations. Preview frame (640x360) 0.556 -> 0.536 ms, textured room (333x217x9) 0.647 -> 0.631 ms, with
+    // the one-warp advance kernel.
     __device__ __forceinline__ void phase_begin(Counters* c, int phase)
     {
-        if (c != nullptr && threadIdx.x == 0) atomicMin(&c->tStart[phase].v, global_ns());
+        if (c != nullptr && blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&c->tStart[phase].v, global_ns());
     }
     __device__ __forceinline__ void phase_end(Counters* c, int phase)
     {
@@ -748,17 +753,23 @@ namespace pt
         uint32_t* stack = reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + threadIdx.x;
         uint32_t* queue = stack + STACK * stride;
         uint32_t* orderWords = reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + (STACK + kLeafQueue) * stride;
-        for (uint32_t k = threadIdx.x; k < kOrderTableBytes / 4; k += blockDim.x)
+        Counters* ctr = work.counters();
+        const uint32_t n = work.count();
+        // (a caller's smaller stack is a test of the lane path's bound)
+        const bool few = work.stackCap == 0 && n <= kFewRays * ((gridDim.x * blockDim.x) >> 5);
+        if (few && blockIdx.x * (blockDim.x >> 5) >= n) return;
+        phase_begin(ctr, Work::kPhase);
+        if (!few)
         {
-            uint32_t w = 0;
-            for (uint32_t b = 0; b < 4; b++) w |= permute_mask((k * 4 + b) & 0xFFu, k >> 6) << (8 * b);
-            orderWords[k] = w;
+            for (uint32_t k = threadIdx.x; k < kOrderTableBytes / 4; k += blockDim.x)
+            {
+                uint32_t w = 0;
+                for (uint32_t b = 0; b < 4; b++) w |= permute_mask((k * 4 + b) & 0xFFu, k >> 6) << (8 * b);
+                orderWords[k] = w;
+            }
+            __syncthreads();
         }
         const uint8_t* slotOrder = reinterpret_cast<const uint8_t*>(orderWords);
-        __syncthreads();
-        Counters* ctr = work.counters();
-        phase_begin(ctr, Work::kPhase);
-        const uint32_t n = work.count();
         const int cap = (work.stackCap > 0 && work.stackCap < STACK) ? work.stackCap : STACK;
         uint32_t visits = 0, tests = 0;  // traversal work of the lane
         const uint32_t lane = lane_id();
@@ -768,8 +779,6 @@ namespace pt
         int waiting = 0;
         bool active = false;     // a ray in flight (finished or not)
         bool exhausted = false;
-        // (a caller's smaller stack is a test of the lane path's bound)
-        const bool few = work.stackCap == 0 && n <= kFewRays * ((gridDim.x * blockDim.x) >> 5);
         if (few)
             trace_few<STACK, ANY>(work, n, reinterpret_cast<uint32_t*>(smem4 + 2u * blockDim.x) + (threadIdx.x >> 5) * 32u * STACK, visits, tests);
         else for (;;)
@@ -842,21 +851,30 @@ namespace pt
                 } while (__popc(holding) * 2 > __popc(busy));
             }
         }
-        if (ctr != nullptr)
+        if (ctr == nullptr) return;
+        unsigned long long v = visits, t = tests;
+        for (int o = 16; o > 0; o >>= 1)
         {
-            unsigned long long v = visits, t = tests;
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-                t += __shfl_down_sync(0xFFFFFFFFu, t, o);
-            }
-            if (lane == 0)
-            {
-                atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, v);
-                atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, t);
-            }
+            v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+            t += __shfl_down_sync(0xFFFFFFFFu, t, o);
         }
-        phase_end(ctr, Work::kPhase);
+        // the block's sums, through the slots of the warps' first lanes
+        unsigned long long* sums = reinterpret_cast<unsigned long long*>(smem4);
+        if (lane == 0)
+        {
+            sums[4u * threadIdx.x] = v;
+            sums[4u * threadIdx.x + 1u] = t;
+        }
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+        for (uint32_t k = 32; k < blockDim.x; k += 32)
+        {
+            v += sums[4u * k];
+            t += sums[4u * k + 1u];
+        }
+        if (v != 0) atomicAdd(&ctr->nodeVisits[ANY ? 1 : 0].v, v);
+        if (t != 0) atomicAdd(&ctr->triTests[ANY ? 1 : 0].v, t);
+        atomicMax(&ctr->tEnd[Work::kPhase].v, global_ns());
     }
 
     // ------------------------------------------------------------------ random numbers
@@ -1573,8 +1591,9 @@ namespace pt
     __global__ void __launch_bounds__(128) shade_kernel(SceneView sc, Wavefront wf, const JobView* jobs, const SceneEntry* scenes)
     {
         Counters* ctr = wf.ctr;
-        phase_begin(ctr, 1);
         const uint32_t n = ctr->matCount[MODEL].v;
+        if (blockIdx.x * blockDim.x >= n) return;
+        phase_begin(ctr, 1);
         const uint32_t cur = ctr->cur;
         const uint32_t nxt = cur ^ 1u;
         const float4* queue = wf.matQ[MODEL];
@@ -1827,55 +1846,94 @@ namespace pt
         phase_end(ctr, 3);
     }
 
+    // What one warp of an iteration's last kernel reads of the counters, each counter by its own lane so that the
+    // loads are in flight together (one after another they took a thread about 5 us).
+    struct IterationCounts
+    {
+        uint32_t own;      // the lane's: [0, 6) hits of the model, 6 and 7 rays of queue 0 and 1, 8 shadow rays, 9 paths shading ended
+        uint32_t cur, rays, next, shadows, ended;
+    };
+    __device__ __forceinline__ IterationCounts iteration_counts(const Wavefront& wf)
+    {
+        static_assert(kModelCount == 6, "lanes of the counters");
+        const Counters* c = wf.ctr;
+        const uint32_t lane = lane_id();
+        IterationCounts k;
+        const uint32_t* p = lane < 6 ? &c->matCount[lane].v : lane < 8 ? &c->rayCount[lane - 6u].v : lane == 8 ? &c->shadowCount.v : &c->regenCount.v;
+        k.own = lane < 10 ? *p : 0u;
+        k.cur = c->cur;
+        k.rays = __shfl_sync(0xFFFFFFFFu, k.own, 6 + static_cast<int>(k.cur));
+        k.next = __shfl_sync(0xFFFFFFFFu, k.own, 7 - static_cast<int>(k.cur));
+        k.shadows = __shfl_sync(0xFFFFFFFFu, k.own, 8);
+        k.ended = __shfl_sync(0xFFFFFFFFu, k.own, 9);
+        // as finished_paths()
+        if (wf.regenBits != nullptr) k.ended += k.rays - __reduce_add_sync(0xFFFFFFFFu, lane < 6 ? k.own : 0u);
+        return k;
+    }
+
+    // Phase times into their sums, and the counters' values for the next iteration. Called by one warp.
+    __device__ __forceinline__ void reset_iteration(Counters* c, const IterationCounts& k, uint32_t next)
+    {
+        const uint32_t lane = lane_id();
+        if (lane < 4)
+        {
+            const unsigned long long start = c->tStart[lane].v, end = c->tEnd[lane].v;
+            if (end > start && start != ~0ull) c->tAccum[lane] += end - start;
+            c->tStart[lane].v = ~0ull;
+            c->tEnd[lane].v = 0;
+        }
+        if (lane < 6) c->matCount[lane].v = 0;
+        else if (lane < 8) c->rayCount[lane - 6u].v = lane - 6u == k.cur ? 0u : next;
+        else if (lane == 8) c->shadowCount.v = 0;
+        else if (lane == 9) c->regenCount.v = 0;
+        else if (lane == 10) c->traceCursor.v = 0;
+        else if (lane == 11) c->shadowCursor.v = 0;
+        else if (lane == 12) c->regenCursor.v = 0;
+        if (lane == 0)
+        {
+            c->raysTraced += k.rays;
+            c->shadowRaysTraced += k.shadows;
+            c->cur = k.cur ^ 1u;
+        }
+    }
+
+    // One warp.
     __global__ void advance_kernel(Wavefront wf, const JobView* jobPtr, cudaGraphConditionalHandle handle, bool graphLoop)
     {
         Counters* c = wf.ctr;
-        const uint32_t cur = c->cur;
-        const uint32_t nxt = cur ^ 1u;
-        const unsigned long long remaining = jobPtr->totalSamples - c->launched;
-        const uint32_t ended = finished_paths(wf);
-        const uint32_t regenerate = static_cast<uint32_t>(remaining < ended ? remaining : ended);
-        const uint32_t next = c->rayCount[nxt].v + regenerate;
-        if (c->iteration < wf.logCapacity)
+        const uint32_t lane = lane_id();
+        const bool cancelled = lane == 0 && wf.cancel != nullptr && *wf.cancel != 0u;
+        const unsigned long long launched = c->launched;
+        const unsigned long long remaining = jobPtr->totalSamples - launched;
+        const uint32_t iteration = c->iteration, maxIterations = jobPtr->maxIterations;
+        const IterationCounts k = iteration_counts(wf);
+        const uint32_t regenerate = static_cast<uint32_t>(remaining < k.ended ? remaining : k.ended);
+        const uint32_t next = k.next + regenerate;
+        if (iteration < wf.logCapacity)
         {
-            uint32_t* row = wf.queueLog + static_cast<size_t>(c->iteration) * kQueueLogColumns;
-            row[0] = c->rayCount[cur].v;
-            for (uint32_t m = 0; m < kModelCount; m++) row[1 + m] = c->matCount[m].v;
-            row[7] = c->shadowCount.v;
-            row[8] = ended;
+            uint32_t* row = wf.queueLog + static_cast<size_t>(iteration) * kQueueLogColumns;
+            if (lane < 6) row[1 + lane] = k.own;
+            else if (lane == 6) row[0] = k.rays;
+            else if (lane == 7) row[7] = k.shadows;
+            else if (lane == 8) row[8] = k.ended;
         }
-        c->raysTraced += c->rayCount[cur].v;
-        c->shadowRaysTraced += c->shadowCount.v;
-        for (int p = 0; p < 4; p++)
-        {
-            if (c->tEnd[p].v > c->tStart[p].v && c->tStart[p].v != ~0ull) c->tAccum[p] += c->tEnd[p].v - c->tStart[p].v;
-            c->tStart[p].v = ~0ull;
-            c->tEnd[p].v = 0;
-        }
-        c->launched += regenerate;
-        c->rayCount[cur].v = 0;
-        c->rayCount[nxt].v = next;
-        c->cur = nxt;
-        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m].v = 0;
-        c->shadowCount.v = 0;
-        c->regenCount.v = 0;
-        c->traceCursor.v = 0;
-        c->shadowCursor.v = 0;
-        c->regenCursor.v = 0;
-        c->iteration += 1;
-        const bool cancelled = wf.cancel != nullptr && *wf.cancel != 0u;
+        reset_iteration(c, k, next);
+        if (lane != 0) return;
+        c->launched = launched + regenerate;
+        c->iteration = iteration + 1u;
         // Every path ends within depthLimit iterations, so the frame needs at most
         // depthLimit * (ceil(samples / pool) + 2) iterations; the cap turns a logic error
         // into an error flag instead of an endless device loop.
-        const bool capped = c->iteration >= jobPtr->maxIterations;
+        const bool capped = iteration + 1u >= maxIterations;
         if (capped && next != 0) c->errorFlags |= kErrIterationCap;
-        c->done = (next == 0 || cancelled || capped) ? 1u : 0u;
+        const bool done = next == 0 || cancelled || capped;
+        c->done = done ? 1u : 0u;
         if (wf.progress != nullptr)
         {
-            wf.progress[0] = c->launched;
-            wf.progress[1] = c->iteration;
+            wf.progress[0] = launched + regenerate;
+            wf.progress[1] = iteration + 1u;
         }
-        if (graphLoop) cudaGraphSetConditional(handle, c->done ? 0u : 1u);
+        if (graphLoop) cudaGraphSetConditional(handle, done ? 0u : 1u);
     }
 
     // PostprocessKernel's tonemap (Image.cu:22-54): x/spp, Reinhard, x^(1/2.2), u8 truncation.
@@ -1999,36 +2057,66 @@ namespace pt
         e->stalled = 0;
     }
 
-    // One thread: hands the iteration's idle slots (finished paths + free list) to the active
-    // jobs, oldest first, within each job's ring window.
-    __global__ void plan_kernel(Wavefront wf, EngineView ev)
+    // One block: hands the iteration's idle slots (finished paths + free list) to the active jobs, oldest first,
+    // within each job's ring window. The jobs' states are read by one thread each, kPlanJobs at a time; thread 0
+    // then goes through them in order (reading them itself, one after another, took it about 1 us per job).
+    constexpr uint32_t kPlanJobs = 128;
+
+    __global__ void __launch_bounds__(kPlanJobs) plan_kernel(Wavefront wf, EngineView ev)
     {
+        __shared__ uint64_t endOf[kPlanJobs], launchedOf[kPlanJobs], totalOf[kPlanJobs];
+        __shared__ uint32_t orderOf[kPlanJobs];
+        __shared__ bool activeOf[kPlanJobs], full;
         EngineCtl* e = ev.ctl;
         const uint32_t avail = finished_paths(wf) + e->freeCount;
+        const uint32_t orderCount = e->orderCount;
         uint32_t launch = 0, segments = 0;
         // a job marked kOrderInTurn gets slots only once every marked job before it has launched all
         // its samples (its turn has come), even if an earlier one's pass window holds it back for now
         bool waitTurn = false;
-        for (uint32_t i = 0; i < e->orderCount && launch < avail; i++)
+        if (threadIdx.x == 0) full = avail == 0;
+        for (uint32_t base = 0; base < orderCount; base += kPlanJobs)
         {
-            const uint32_t o = ev.order[i];
-            const uint32_t j = o & ~kOrderInTurn;
-            JobView& J = ev.jobs[j];
-            if (J.state != kJobActive) continue;
-            const bool inTurn = (o & kOrderInTurn) != 0;
-            if (inTurn && waitTurn) continue;
-            const uint64_t end = job_window_end(J);
-            if (end > J.launched)
+            const uint32_t mine = base + threadIdx.x;
+            if (mine < orderCount)
             {
-                const uint64_t can = end - J.launched;
-                const uint32_t take = static_cast<uint32_t>(can < static_cast<uint64_t>(avail - launch) ? can : avail - launch);
-                ev.segments[segments] = LaunchSegment{j, launch, J.launched};
-                segments++;
-                J.launched += take;
-                launch += take;
+                const uint32_t o = ev.order[mine];
+                const JobView& J = ev.jobs[o & ~kOrderInTurn];
+                orderOf[threadIdx.x] = o;
+                activeOf[threadIdx.x] = J.state == kJobActive;
+                endOf[threadIdx.x] = job_window_end(J);
+                launchedOf[threadIdx.x] = J.launched;
+                totalOf[threadIdx.x] = J.totalSamples;
             }
-            if (inTurn && J.launched < J.totalSamples) waitTurn = true;
+            __syncthreads();
+            if (full) break;
+            if (threadIdx.x == 0)
+            {
+                const uint32_t count = orderCount - base < kPlanJobs ? orderCount - base : kPlanJobs;
+                for (uint32_t i = 0; i < count && launch < avail; i++)
+                {
+                    if (!activeOf[i]) continue;
+                    const uint32_t j = orderOf[i] & ~kOrderInTurn;
+                    const bool inTurn = (orderOf[i] & kOrderInTurn) != 0;
+                    if (inTurn && waitTurn) continue;
+                    uint64_t launched = launchedOf[i];
+                    if (endOf[i] > launched)
+                    {
+                        const uint64_t can = endOf[i] - launched;
+                        const uint32_t take = static_cast<uint32_t>(can < static_cast<uint64_t>(avail - launch) ? can : avail - launch);
+                        ev.segments[segments] = LaunchSegment{j, launch, launched};
+                        segments++;
+                        launched += take;
+                        ev.jobs[j].launched = launched;
+                        launch += take;
+                    }
+                    if (inTurn && launched < totalOf[i]) waitTurn = true;
+                }
+                full = launch >= avail;
+            }
+            __syncthreads();
         }
+        if (threadIdx.x != 0) return;
         e->launchCount = launch;
         e->segmentCount = segments;
     }
@@ -2274,32 +2362,17 @@ namespace pt
             }
         }
         __syncthreads();
-        if (threadIdx.x != 0) return;
+        if (threadIdx.x >= 32) return;
         Counters* c = wf.ctr;
         EngineCtl* e = ev.ctl;
-        const uint32_t cur = c->cur;
-        const uint32_t nxt = cur ^ 1u;
+        const bool bell = threadIdx.x == 0 && ev.doorbell != nullptr && *ev.doorbell != 0u;
         const uint32_t launch = e->launchCount;
-        const uint32_t next = c->rayCount[nxt].v + launch;
-        c->raysTraced += c->rayCount[cur].v;
-        c->shadowRaysTraced += c->shadowCount.v;
-        for (int p = 0; p < 4; p++)
-        {
-            if (c->tEnd[p].v > c->tStart[p].v && c->tStart[p].v != ~0ull) c->tAccum[p] += c->tEnd[p].v - c->tStart[p].v;
-            c->tStart[p].v = ~0ull;
-            c->tEnd[p].v = 0;
-        }
-        e->freeCount = e->freeCount + finished_paths(wf) - launch;
+        const IterationCounts k = iteration_counts(wf);
+        const uint32_t next = k.next + launch;
+        reset_iteration(c, k, next);
+        if (threadIdx.x != 0) return;
+        e->freeCount = e->freeCount + k.ended - launch;
         c->launched += launch;
-        c->rayCount[cur].v = 0;
-        c->rayCount[nxt].v = next;
-        c->cur = nxt;
-        for (uint32_t m = 0; m < kModelCount; m++) c->matCount[m].v = 0;
-        c->shadowCount.v = 0;
-        c->regenCount.v = 0;
-        c->traceCursor.v = 0;
-        c->shadowCursor.v = 0;
-        c->regenCursor.v = 0;
         c->iteration += 1;
         e->launchCount = 0;
         e->segmentCount = 0;
@@ -2309,7 +2382,6 @@ namespace pt
         e->sliceIterations += 1;
         const bool idle = next == 0 && !launchable;
         if (idle && unfinished) e->stalled = 1;
-        const bool bell = ev.doorbell != nullptr && *ev.doorbell != 0u;
         c->done = (completed > 0 || bell || idle || e->sliceIterations >= e->maxSliceIterations) ? 1u : 0u;
         if (wf.progress != nullptr)
         {
@@ -2569,7 +2641,7 @@ namespace pt
         else
             regen_kernel<<<L.shadeBlocks, 256, 0, s>>>(L.wf, L.job);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        advance_kernel<<<1, 1, 0, s>>>(L.wf, L.job, L.handle, L.graphLoop);
+        advance_kernel<<<1, 32, 0, s>>>(L.wf, L.job, L.handle, L.graphLoop);
         return cudaGetLastError();
     }
 
@@ -2595,7 +2667,7 @@ namespace pt
             e = launch_trace<true>(ws, L.scene.depth, L.occupancy, L.traceBlocks, L.traceThreads, L.refillShadow, &L.wf.ctr->errorFlags, s);
             if (e != cudaSuccess) return e;
         }
-        plan_kernel<<<1, 1, 0, s>>>(L.wf, L.ev);
+        plan_kernel<<<1, kPlanJobs, 0, s>>>(L.wf, L.ev);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         engine_regen_bits_kernel<<<L.sms * engine_regen_blocks_per_sm(), 256, 0, s>>>(L.wf, L.ev);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -70,8 +70,14 @@ namespace pt
     cudaError_t launch_resolve(const JobView* job, float4* accumulation, uint32_t* framebuffer, int blocks, cudaStream_t stream);
     cudaError_t launch_resolve_fp64(const JobView* job, double* sums, int blocks, cudaStream_t stream);
     cudaError_t launch_clear(uint32_t* framebuffer, uint32_t n, uint32_t value, cudaStream_t stream);
-    cudaError_t launch_batch_trace(const SceneView& scene, uint32_t root, const float* rays, uint32_t n, uint32_t* cursor, uint32_t* triOut,
-                                   float* uvtOut, uint8_t* occOut, int blocks, int threads, uint32_t* errorFlags, cudaStream_t stream,
+    // A ray batch's words on the device, all zero between batches.
+    struct alignas(256) BatchState
+    {
+        uint32_t cursor, errors, left;
+    };
+    // *hostErrors (host-mapped memory) gets the error flags if there are any.
+    cudaError_t launch_batch_trace(const SceneView& scene, uint32_t root, const float* rays, uint32_t n, BatchState* state, uint32_t* hostErrors,
+                                   uint32_t* triOut, float* uvtOut, uint8_t* occOut, int blocks, int threads, cudaStream_t stream,
                                    uint32_t bvhFormat = kBvh8Quantised);
     // models[t] = model of triangle t's material (0 if its index is out of range); *mask: bit m = model m is present,
     // bit kModelCount = an index is out of range.

@@ -12,6 +12,7 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <filesystem>
@@ -344,12 +345,14 @@ namespace pt
             }
             PT_CUDA("cudaEventCreate", cudaEventCreate(&startEvent_));
             PT_CUDA("cudaEventCreate", cudaEventCreate(&stopEvent_));
-            PT_CUDA("cudaHostAlloc", cudaHostAlloc(&hostMapped_, 64, cudaHostAllocMapped));
-            std::memset(hostMapped_, 0, 64);
+            PT_CUDA("cudaHostAlloc", cudaHostAlloc(&hostMapped_, 64 + 4 * kBatchStates, cudaHostAllocMapped));
+            std::memset(hostMapped_, 0, 64 + 4 * kBatchStates);
             PT_CUDA("cudaHostGetDevicePointer", cudaHostGetDevicePointer(&hostMappedDev_, hostMapped_, 0));
             PT_TRY(job_.allocate(sizeof(JobView)));
             PT_TRY(counters_.allocate(sizeof(Counters)));
-            PT_TRY(cursor_.allocate(64));
+            PT_TRY(batches_.allocate(kBatchStates * sizeof(BatchState)));
+            PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(batches_.get<void>(), 0, kBatchStates * sizeof(BatchState), stream_));
+            PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream_));
             return Status::Ok();
         }
 
@@ -840,18 +843,42 @@ namespace pt
             if (!rays || (!occ && (!tri || !uvt))) return Status::Err(GPT_ERR_INVALID_ARGUMENT, "Null ray or output pointer");
             PT_CUDA("cudaSetDevice", cudaSetDevice(device_));
             cudaStream_t st = s ? s : stream_;
-            uint32_t* cursor = cursor_.get<uint32_t>();
-            PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(cursor, 0, 8, st));
             const SceneView sv = scene_->view();
             if (bvh == kBvh2Fp32 && !sv.nodes2) return Status::Err(GPT_ERR_STATE, "The scene has no binary BVH");
             const int blocks = trace_grid_blocks(device_, 128, sv.depth, kBatchOccupancy, bvh);
-            PT_CUDA("intersect", launch_batch_trace(sv, 0u, rays, n, cursor, tri, uvt, occ, blocks, 128, cursor + 1, st, bvh));
-            uint32_t err = 0;
-            PT_CUDA("cudaMemcpyAsync", cudaMemcpyAsync(&err, cursor + 1, 4, cudaMemcpyDeviceToHost, st));
+            const BatchSlot slot(*this);
+            volatile uint32_t* errors = reinterpret_cast<volatile uint32_t*>(static_cast<char*>(hostMapped_) + 64) + slot.index;
+            uint32_t* errorsDev = reinterpret_cast<uint32_t*>(static_cast<char*>(hostMappedDev_) + 64) + slot.index;
+            *errors = 0u;
+            PT_CUDA("intersect", launch_batch_trace(sv, 0u, rays, n, batches_.get<BatchState>() + slot.index, errorsDev, tri, uvt, occ, blocks, 128, st, bvh));
             PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(st));
-            if (err) return Status::Err(GPT_ERR_DEVICE_FAULT, "Traversal reported error flags " + std::to_string(err));
+            if (*errors) return Status::Err(GPT_ERR_DEVICE_FAULT, "Traversal reported error flags " + std::to_string(*errors));
             return Status::Ok();
         }
+
+        // One of the batch states, for one call: callers on several threads get different ones.
+        struct BatchSlot
+        {
+            Renderer& impl;
+            uint32_t index;
+            explicit BatchSlot(Renderer& i) : impl(i)
+            {
+                std::unique_lock lock(impl.batchMutex_);
+                impl.batchFreed_.wait(lock, [&] { return impl.batchesFree_ != 0; });
+                index = static_cast<uint32_t>(__builtin_ctz(impl.batchesFree_));
+                impl.batchesFree_ &= impl.batchesFree_ - 1u;
+            }
+            ~BatchSlot()
+            {
+                {
+                    std::scoped_lock lock(impl.batchMutex_);
+                    impl.batchesFree_ |= 1u << index;
+                }
+                impl.batchFreed_.notify_one();
+            }
+            BatchSlot(const BatchSlot&) = delete;
+            BatchSlot& operator=(const BatchSlot&) = delete;
+        };
 
         // ---------------------------------------------------------------- simulation thread
         Status StartSimulation(uint32_t width, uint32_t height, float fovY, const gpt_motion_state* states, uint32_t count, uint32_t spp,
@@ -988,12 +1015,16 @@ namespace pt
         cudaEvent_t shadeJoin_[kModelCount] = {};
         cudaStream_t shadeStreams_[kModelCount] = {};
         void* hostMapped_ = nullptr;
-        void* hostMappedDev_ = nullptr;
+        void* hostMappedDev_ = nullptr;  // [0] cancel flag, [16] progress, [32] loop condition, [64] error flags of the batch states
+        static constexpr uint32_t kBatchStates = 16;
+        std::mutex batchMutex_;
+        std::condition_variable batchFreed_;
+        uint32_t batchesFree_ = (1u << kBatchStates) - 1u;
         static constexpr uint32_t kDefaultPool = 1u << 20;
         static constexpr uint32_t kLogCapacity = 1u << 16;
         uint32_t pool_ = 0;
         DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regen_, regenBits_, slotT_, slotL_, slotSample_, queueLog_;
-        DeviceBuffer counters_, job_, cursor_, accumulation_, framebuffer_, sampleRadiance_;
+        DeviceBuffer counters_, job_, batches_, accumulation_, framebuffer_, sampleRadiance_;
         JobView hostJob_{};
         Counters hostCounters_{};
         std::unique_ptr<SceneGpu> scene_;

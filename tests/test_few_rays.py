@@ -34,3 +34,37 @@ def test_batches_equal_the_binary_bvh(gpu_renderer, scene_factory, name, n):
         assert np.array_equal(t8, tri) and np.array_equal(u8.view(np.uint32), uvt.view(np.uint32))
         assert np.array_equal(r.trace_any_np(rays), occ)
     r.set_bvh_build(pathtracer.BVH_BUILD_HOST)
+
+
+@pytest.mark.gpu
+def test_batches_of_several_threads(gpu_renderer, scene_factory):
+    """20 threads with streams of their own on one renderer (16 batches can be in flight) and batches of both kinds."""
+    import threading
+    import torch
+    s = scene_factory("spheres-10k")
+    r = gpu_renderer
+    r.upload_scene(s)
+    batches = []
+    for n in (1, 700, 30001):
+        rays = ray_mix(s, n)
+        batches.append((torch.from_numpy(rays).cuda(),) + r.trace_closest_np(rays))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for i in range(12):
+                rays, tri, uvt = batches[(i + k) % 3]
+                t = torch.empty(rays.shape[0], dtype=torch.int32, device="cuda")
+                u = torch.empty((rays.shape[0], 3), dtype=torch.float32, device="cuda")
+                r.intersect_closest(rays, t, u, stream=stream.cuda_stream)
+                if not (np.array_equal(t.cpu().numpy().view(np.uint32), tri) and np.array_equal(u.cpu().numpy(), uvt)):
+                    wrong.append((k, i))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(20)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

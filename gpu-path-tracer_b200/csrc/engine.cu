@@ -306,8 +306,7 @@ namespace pt
             PT_TRY(shL_.allocate(P * 16));
             PT_TRY(regenBits_.allocate((P + 31) / 32 * 4));
             PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(regenBits_.get<void>(), 0, (P + 31) / 32 * 4, stream_));
-            PT_TRY(slotT_.allocate(P * 16));
-            PT_TRY(slotL_.allocate(P * 16));
+            PT_TRY(slots_.allocate(P * 32));
             PT_TRY(slotSample_.allocate(P * 4));
             PT_TRY(freeList_.allocate(P * 4));
             PT_TRY(counters_.allocate(sizeof(Counters)));
@@ -539,8 +538,7 @@ namespace pt
             w.shD = shD_.get<float4>();
             w.shL = shL_.get<float4>();
             w.regenBits = regenBits_.get<uint32_t>();  // the engine always regenerates from the bitmap
-            w.slotT = slotT_.get<float4>();
-            w.slotL = slotL_.get<float4>();
+            w.slots = slots_.get<float4>();
             w.slotSample = slotSample_.get<uint32_t>();
             w.capacity = cfg_.pool_size;
             w.logCapacity = 0;
@@ -1034,7 +1032,7 @@ namespace pt
         JobView* mirror_ = nullptr;
         uint32_t* orderHost_ = nullptr;
         uint32_t* sliceWords_ = nullptr;
-        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regenBits_, slotT_, slotL_, slotSample_, freeList_;
+        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regenBits_, slots_, slotSample_, freeList_;
         DeviceBuffer counters_, ctl_, jobs_, order_, segments_;
         ScenePack pack_;
         PinnedUpload upload_;

@@ -273,8 +273,7 @@ namespace pt
         float4* shL;
         uint32_t* regen;
         uint32_t* regenBits;      // bit per slot set when its path finished (nullptr: the regen queue, frame renderer only)
-        float4* slotT;            // throughput xyz, w = bits(depth | delta << 8)
-        float4* slotL;            // radiance xyz, w = bits(rng stream position)
+        float4* slots;            // per slot: throughput xyz, bits(depth | delta << 8); radiance xyz, bits(rng stream position)
         uint32_t* slotSample;
         uint32_t capacity;
         uint32_t logCapacity;

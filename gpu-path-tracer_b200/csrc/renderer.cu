@@ -384,7 +384,7 @@ namespace pt
 
         Status ensurePool(uint32_t pool)
         {
-            if (pool == pool_ && slotT_.get<float4>()) return Status::Ok();
+            if (pool == pool_ && slots_.get<float4>()) return Status::Ok();
             releaseGraph();
             const size_t P = pool;
             for (int q = 0; q < 2; q++)
@@ -399,8 +399,7 @@ namespace pt
             PT_TRY(regen_.allocate(P * 4));
             PT_TRY(regenBits_.allocate((P + 31) / 32 * 4));
             PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(regenBits_.get<void>(), 0, (P + 31) / 32 * 4, stream_));
-            PT_TRY(slotT_.allocate(P * 16));
-            PT_TRY(slotL_.allocate(P * 16));
+            PT_TRY(slots_.allocate(P * 32));
             PT_TRY(slotSample_.allocate(P * 4));
             PT_TRY(queueLog_.allocate(static_cast<size_t>(kLogCapacity) * kQueueLogColumns * 4));
             pool_ = pool;
@@ -421,8 +420,7 @@ namespace pt
             w.shL = shL_.get<float4>();
             w.regen = regen_.get<uint32_t>();
             w.regenBits = queues ? nullptr : regenBits_.get<uint32_t>();
-            w.slotT = slotT_.get<float4>();
-            w.slotL = slotL_.get<float4>();
+            w.slots = slots_.get<float4>();
             w.slotSample = slotSample_.get<uint32_t>();
             w.capacity = pool_;
             w.logCapacity = kLogCapacity;
@@ -1023,7 +1021,7 @@ namespace pt
         static constexpr uint32_t kDefaultPool = 1u << 20;
         static constexpr uint32_t kLogCapacity = 1u << 16;
         uint32_t pool_ = 0;
-        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regen_, regenBits_, slotT_, slotL_, slotSample_, queueLog_;
+        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regen_, regenBits_, slots_, slotSample_, queueLog_;
         DeviceBuffer counters_, job_, batches_, accumulation_, framebuffer_, sampleRadiance_;
         JobView hostJob_{};
         Counters hostCounters_{};

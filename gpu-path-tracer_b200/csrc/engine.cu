@@ -297,12 +297,10 @@ namespace pt
             const size_t P = cfg_.pool_size;
             for (int q = 0; q < 2; q++)
             {
-                PT_TRY(rayO_[q].allocate(P * 16));
-                PT_TRY(rayD_[q].allocate(P * 16));
+                PT_TRY(rays_[q].allocate(P * 32));
             }
             PT_TRY(matQ_.allocate(P * 48 * kModelCount));
-            PT_TRY(shO_.allocate(P * 16));
-            PT_TRY(shD_.allocate(P * 16));
+            PT_TRY(shRays_.allocate(P * 32));
             PT_TRY(shL_.allocate(P * 16));
             PT_TRY(regenBits_.allocate((P + 31) / 32 * 4));
             PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(regenBits_.get<void>(), 0, (P + 31) / 32 * 4, stream_));
@@ -530,12 +528,14 @@ namespace pt
             Wavefront w{};
             for (int q = 0; q < 2; q++)
             {
-                w.rayO[q] = rayO_[q].get<float4>();
-                w.rayD[q] = rayD_[q].get<float4>();
+                w.rays[q] = rays_[q].get<float4>();
             }
-            for (uint32_t m = 0; m < kModelCount; m++) w.matQ[m] = matQ_.get<float4>() + size_t(m) * cfg_.pool_size * 3;
-            w.shO = shO_.get<float4>();
-            w.shD = shD_.get<float4>();
+            for (uint32_t m = 0; m < kModelCount; m++)
+            {
+                w.matQ[m] = matQ_.get<float4>() + size_t(m) * cfg_.pool_size * 2;
+                w.matHit[m] = matQ_.get<float4>() + (size_t(kModelCount) * 2 + m) * cfg_.pool_size;
+            }
+            w.shRays = shRays_.get<float4>();
             w.shL = shL_.get<float4>();
             w.regenBits = regenBits_.get<uint32_t>();  // the engine always regenerates from the bitmap
             w.slots = slots_.get<float4>();
@@ -1032,7 +1032,7 @@ namespace pt
         JobView* mirror_ = nullptr;
         uint32_t* orderHost_ = nullptr;
         uint32_t* sliceWords_ = nullptr;
-        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regenBits_, slots_, slotSample_, freeList_;
+        DeviceBuffer rays_[2], matQ_, shRays_, shL_, regenBits_, slots_, slotSample_, freeList_;
         DeviceBuffer counters_, ctl_, jobs_, order_, segments_;
         ScenePack pack_;
         PinnedUpload upload_;

@@ -79,6 +79,21 @@ namespace pt
             : "l"(p));
     }
 
+    // 32 bytes of memory that kernels write (32-byte aligned). Queue entries are 32-byte records (and 16 bytes more
+    // for hits and shadow radiance), which halves the accesses of refilling and retiring rays against arrays of
+    // float4: spheres-1m frame (1920x1080x64) closest hits 36.3 -> 35.8 ms, regeneration 4.56 -> 4.46 ms.
+    __device__ __forceinline__ void load8(const float4* p, float4& a, float4& b)
+    {
+        asm("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+            : "l"(p));
+    }
+    __device__ __forceinline__ void store8(float4* p, float4 a, float4 b)
+    {
+        asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+            :: "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p) : "memory");
+    }
+
     // ------------------------------------------------------------------ traversal
     // Registers of a ray in flight. Values a traversal step reads rarely live in the thread's slot
     // of shared memory instead (ColdSlot), which keeps the node test free of register spills.
@@ -331,17 +346,8 @@ namespace pt
     // shading 0.975 -> 0.895 ms.
     __device__ __forceinline__ float4& slot_throughput(const Wavefront& wf, uint32_t slot) { return wf.slots[2u * static_cast<size_t>(slot)]; }
     __device__ __forceinline__ float4& slot_radiance(const Wavefront& wf, uint32_t slot) { return wf.slots[2u * static_cast<size_t>(slot) + 1u]; }
-    __device__ __forceinline__ void load_slot(const Wavefront& wf, uint32_t slot, float4& T, float4& L)
-    {
-        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-            : "=f"(T.x), "=f"(T.y), "=f"(T.z), "=f"(T.w), "=f"(L.x), "=f"(L.y), "=f"(L.z), "=f"(L.w)
-            : "l"(&slot_throughput(wf, slot)) : "memory");
-    }
-    __device__ __forceinline__ void store_slot(const Wavefront& wf, uint32_t slot, float4 T, float4 L)
-    {
-        asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
-            :: "f"(T.x), "f"(T.y), "f"(T.z), "f"(T.w), "f"(L.x), "f"(L.y), "f"(L.z), "f"(L.w), "l"(&slot_throughput(wf, slot)) : "memory");
-    }
+    __device__ __forceinline__ void load_slot(const Wavefront& wf, uint32_t slot, float4& T, float4& L) { load8(&slot_throughput(wf, slot), T, L); }
+    __device__ __forceinline__ void store_slot(const Wavefront& wf, uint32_t slot, float4 T, float4 L) { store8(&slot_throughput(wf, slot), T, L); }
 
     // A path left its slot: recorded for regeneration, in the finished-slot bitmap or (the reference's
     // structure) in the regeneration queue. With the bitmap the caller counts: finished_paths().
@@ -387,7 +393,8 @@ namespace pt
         __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& tag) const
         {
             const uint32_t cur = wf.ctr->cur;
-            const float4 a = wf.rayO[cur][i], b = wf.rayD[cur][i];
+            float4 a, b;
+            load8(wf.rays[cur] + 2u * static_cast<size_t>(i), a, b);
             o = make_float3(a.x, a.y, a.z);
             d = make_float3(b.x, b.y, b.z);
             tmin = kMinT;
@@ -401,10 +408,9 @@ namespace pt
             if (h.tri != kInvalid)
             {
                 const uint32_t pos = agg_push_keyed(wf.ctr->matCount, h.model);
-                float4* e = wf.matQ[h.model] + static_cast<size_t>(pos) * 3;
-                e[0] = make_float4(o.x, o.y, o.z, __uint_as_float(tag));
-                e[1] = make_float4(d.x, d.y, d.z, kMaxT);
-                e[2] = make_float4(__uint_as_float(h.tri), h.u, h.v, h.t);
+                store8(wf.matQ[h.model] + 2u * static_cast<size_t>(pos), make_float4(o.x, o.y, o.z, __uint_as_float(tag)),
+                       make_float4(d.x, d.y, d.z, __uint_as_float(h.tri)));
+                wf.matHit[h.model][pos] = make_float4(0.0f, h.u, h.v, h.t);
             }
             else
             {
@@ -437,7 +443,8 @@ namespace pt
         __device__ uint32_t* cursor() const { return &wf.ctr->shadowCursor.v; }
         __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& tag) const
         {
-            const float4 a = wf.shO[i], b = wf.shD[i];
+            float4 a, b;
+            load8(wf.shRays + 2u * static_cast<size_t>(i), a, b);
             o = make_float3(a.x, a.y, a.z);
             d = make_float3(b.x, b.y, b.z);
             tmin = kMinT;
@@ -1060,8 +1067,8 @@ namespace pt
         store_slot(wf, slot, make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(pack_meta(0, true, jobIndex))),
                    make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(4u)));
         wf.slotSample[slot] = sample;
-        wf.rayO[queue][position] = make_float4(o.x, o.y, o.z, __uint_as_float(slot | (job.scene << kSlotBits)));
-        wf.rayD[queue][position] = make_float4(d.x, d.y, d.z, kMaxT);
+        store8(wf.rays[queue] + 2u * static_cast<size_t>(position), make_float4(o.x, o.y, o.z, __uint_as_float(slot | (job.scene << kSlotBits))),
+               make_float4(d.x, d.y, d.z, kMaxT));
     }
 
     __global__ void frame_init_kernel(Wavefront wf, const JobView* job, uint32_t pool)
@@ -1653,15 +1660,14 @@ namespace pt
             float4 shOut0 = rayOut0, shOut1 = rayOut0, shOut2 = rayOut0;
             if (k < n)
             {
-                const float4* entry = queue + static_cast<size_t>(k) * 3;
-                const float4 o4 = entry[0];
-                const float4 d4 = entry[1];
-                const float4 h4 = entry[2];
+                float4 o4, d4;
+                load8(queue + 2u * static_cast<size_t>(k), o4, d4);
+                const float4 h4 = wf.matHit[MODEL][k];
                 const uint32_t tag = __float_as_uint(o4.w);
                 const uint32_t slot = tag & kSlotMask;
                 const float3 o = f3(o4), d = f3(d4);
                 const float tHit = h4.w;
-                const uint32_t tri = __float_as_uint(h4.x);
+                const uint32_t tri = __float_as_uint(d4.w);
                 float4 T4, L4;
                 load_slot(wf, slot, T4, L4);
                 const uint32_t meta = __float_as_uint(T4.w);
@@ -1851,14 +1857,12 @@ namespace pt
             if (pushRay)
             {
                 const uint32_t pos = blockBase[0] + octBase[oct] + rank;
-                wf.rayO[nxt][pos] = rayOut0;
-                wf.rayD[nxt][pos] = rayOut1;
+                store8(wf.rays[nxt] + 2u * static_cast<size_t>(pos), rayOut0, rayOut1);
             }
             if (pushShadow)
             {
                 const uint32_t pos = blockBase[1] + octBase[soct] + srank;
-                wf.shO[pos] = shOut0;
-                wf.shD[pos] = shOut1;
+                store8(wf.shRays + 2u * static_cast<size_t>(pos), shOut0, shOut1);
                 wf.shL[pos] = shOut2;
             }
             __syncthreads();

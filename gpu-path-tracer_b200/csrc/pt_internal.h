@@ -8,8 +8,8 @@
 //   alias bin         16 B  q, p, alias, value (AliasTableView.hpp:8-14); two tables, area and power weights
 //   path slot         36 B  throughput|depth/flags/job, radiance|rng position, sample index
 //   ray queue entry   32 B  origin|tag, direction|tMax   (x2, ping-pong; tag = slot | scene << 24)
-//   material queue    48 B  origin|tag, direction|tMax, triangle|u|v|t   (x6, one per shading model: the
-//                           closest-hit kernel writes the ray and its hit, so shading reads one entry)
+//   material queue    48 B  origin|tag, direction|triangle (32 B) and -|u|v|t (16 B)   (x6, one per shading
+//                           model: the closest-hit kernel writes the ray and its hit, so shading reads one entry)
 //   shadow queue      48 B  origin|slot, direction|tMax, radiance
 //   regen queue        4 B  slot
 #pragma once
@@ -265,11 +265,10 @@ namespace pt
 
     struct Wavefront
     {
-        float4* rayO[2];
-        float4* rayD[2];
-        float4* matQ[kModelCount];   // per model: entries of 3 float4 = origin|tag, direction|tMax, triangle|u|v|t
-        float4* shO;
-        float4* shD;
+        float4* rays[2];             // entries of 2 float4 = origin|tag, direction|tMax
+        float4* matQ[kModelCount];   // per model: entries of 2 float4 = origin|tag, direction|triangle
+        float4* matHit[kModelCount]; // and -|u|v|t
+        float4* shRays;              // as rays
         float4* shL;
         uint32_t* regen;
         uint32_t* regenBits;      // bit per slot set when its path finished (nullptr: the regen queue, frame renderer only)

@@ -389,12 +389,10 @@ namespace pt
             const size_t P = pool;
             for (int q = 0; q < 2; q++)
             {
-                PT_TRY(rayO_[q].allocate(P * 16));
-                PT_TRY(rayD_[q].allocate(P * 16));
+                PT_TRY(rays_[q].allocate(P * 32));
             }
             PT_TRY(matQ_.allocate(P * 48 * kModelCount));
-            PT_TRY(shO_.allocate(P * 16));
-            PT_TRY(shD_.allocate(P * 16));
+            PT_TRY(shRays_.allocate(P * 32));
             PT_TRY(shL_.allocate(P * 16));
             PT_TRY(regen_.allocate(P * 4));
             PT_TRY(regenBits_.allocate((P + 31) / 32 * 4));
@@ -411,12 +409,14 @@ namespace pt
             Wavefront w{};
             for (int q = 0; q < 2; q++)
             {
-                w.rayO[q] = rayO_[q].get<float4>();
-                w.rayD[q] = rayD_[q].get<float4>();
+                w.rays[q] = rays_[q].get<float4>();
             }
-            for (uint32_t m = 0; m < kModelCount; m++) w.matQ[m] = matQ_.get<float4>() + static_cast<size_t>(m) * pool_ * 3;
-            w.shO = shO_.get<float4>();
-            w.shD = shD_.get<float4>();
+            for (uint32_t m = 0; m < kModelCount; m++)
+            {
+                w.matQ[m] = matQ_.get<float4>() + static_cast<size_t>(m) * pool_ * 2;
+                w.matHit[m] = matQ_.get<float4>() + (static_cast<size_t>(kModelCount) * 2 + m) * pool_;
+            }
+            w.shRays = shRays_.get<float4>();
             w.shL = shL_.get<float4>();
             w.regen = regen_.get<uint32_t>();
             w.regenBits = queues ? nullptr : regenBits_.get<uint32_t>();
@@ -1021,7 +1021,7 @@ namespace pt
         static constexpr uint32_t kDefaultPool = 1u << 20;
         static constexpr uint32_t kLogCapacity = 1u << 16;
         uint32_t pool_ = 0;
-        DeviceBuffer rayO_[2], rayD_[2], matQ_, shO_, shD_, shL_, regen_, regenBits_, slots_, slotSample_, queueLog_;
+        DeviceBuffer rays_[2], matQ_, shRays_, shL_, regen_, regenBits_, slots_, slotSample_, queueLog_;
         DeviceBuffer counters_, job_, batches_, accumulation_, framebuffer_, sampleRadiance_;
         JobView hostJob_{};
         Counters hostCounters_{};

@@ -5,7 +5,7 @@
 //   shade_kernel<model>    one launch per shading model present (MaterialEval.cu:194-912)
 //   trace_kernel<any>      NEE shadow rays, any hit; unoccluded radiance added to the path slot
 //   regen_bits_kernel      finished paths -> per-sample radiance; new samples -> next ray queue
-//   advance_kernel         one thread: queue bookkeeping, log, loop condition (Renderer.cpp:573-619)
+//   advance_kernel         one warp: queue bookkeeping, log, loop condition (Renderer.cpp:573-619)
 // Every expression that reaches a result is written in the reference's operator order. The
 // product library compiles this file as the reference's kernels are compiled (multiply-add
 // contraction, CUDA's sinf/cosf/powf/rsqrtf); the deterministic library compiles it with
@@ -146,7 +146,7 @@ namespace pt
             }
             else if (hit)
             {
-                // better_hit with the best triangle read from shared memory: it matters only at a tie
+                // the nearest hit, the smaller input index at a tie (only then the best triangle is read from shared memory)
                 if (t >= tmin && t <= st.hitT)
                 {
                     const uint32_t orig = __float_as_uint(a.w);

@@ -217,11 +217,4 @@ namespace pt
         float u, v;
         uint32_t model;
     };
-
-    // Closest-hit acceptance with the deterministic tie rule: the smaller input index wins
-    // at a bit-identical t.
-    PT_HD bool better_hit(float t, uint32_t orig, float tmin, float bestT, uint32_t bestTri)
-    {
-        return t >= tmin && (t < bestT || (t == bestT && bestTri != kInvalid && orig < bestTri));
-    }
 }

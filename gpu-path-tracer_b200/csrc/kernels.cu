@@ -385,6 +385,7 @@ namespace pt
         int stackCap = 0;          // traversal stack entries a ray may use (0 = the kernel's whole stack)
         static constexpr int kPhase = 0;
         static constexpr bool kBatch = false;
+        static constexpr uint32_t kFewRays = 4;
         static constexpr bool kFixedTmin = true;   // every wavefront ray starts at kMinT
         __device__ uint32_t root(uint32_t tag) const { return scenes ? __ldg(&scenes[tag >> kSlotBits].root) : 0u; }
         __device__ Counters* counters() const { return wf.ctr; }
@@ -436,6 +437,7 @@ namespace pt
         int stackCap = 0;
         static constexpr int kPhase = 2;
         static constexpr bool kBatch = false;
+        static constexpr uint32_t kFewRays = 4;
         static constexpr bool kFixedTmin = true;
         __device__ uint32_t root(uint32_t tag) const { return scenes ? __ldg(&scenes[tag >> kSlotBits].root) : 0u; }
         __device__ Counters* counters() const { return wf.ctr; }
@@ -479,6 +481,7 @@ namespace pt
         int stackCap = 0;
         static constexpr int kPhase = 0;
         static constexpr bool kBatch = true;
+        static constexpr uint32_t kFewRays = 8;
         static constexpr bool kFixedTmin = false;  // per-ray tMin of the caller's batch
         __device__ uint32_t root(uint32_t) const { return rootNode; }
         __device__ Counters* counters() const { return nullptr; }
@@ -636,10 +639,12 @@ namespace pt
     // took about 35 us per launch. Here up to 4 nodes off the top of the ray's stack are visited at once, each by
     // 8 lanes that test a child each, and the triangles of all their leaves at once; nodes behind the closest hit
     // are dropped. 640x360 preview frame of spheres-200k: 0.80 -> 0.54 ms on the device; textured room 333x217x9:
-    // 0.72 -> 0.64 ms; large frames 0.4 ms. Up to kFewRays rays per warp of the grid: 2 took the preview 0.60 ms,
-    // 8 the same as 4, 16 slowed the Cornell box frame from 3.38 to 3.48 ms. (8 lanes per ray and one node at a
-    // time, for 32 to 64 rays per warp, was slower than a lane per ray: preview 0.64 to 0.69 ms.)
-    constexpr uint32_t kFewRays = 4;
+    // 0.72 -> 0.64 ms; large frames 0.4 ms. Up to Work::kFewRays rays per warp of the grid. In a frame 4: 2 took the
+    // preview 0.60 ms, 8 the same as 4, 16 slowed the Cornell box frame from 3.38 to 3.48 ms. In a batch, whose rays
+    // are less coherent than those of most iterations, 8: 42,001 closest-hit rays took 46, 58 and 82 us with it and
+    // 47, 68 and 93 us with a lane per ray (10K, 205K and 1.31M triangles; any-hit rays 43, 56, 59 and 43, 56, 70 us),
+    // and with 16, 84,001 rays 68, 93 and 129 us against 49, 69 and 94. (8 lanes per ray and one node at a time, for
+    // 32 to 64 rays per warp, was slower than a lane per ray: preview 0.64 to 0.69 ms.)
     constexpr int kFewNodes = 4;
 
     // stack: 32 * STACK words of the warp: 16 * STACK records and as many entry distances. From at most
@@ -804,7 +809,7 @@ namespace pt
         Counters* ctr = work.counters();
         const uint32_t n = work.count();
         // (a caller's smaller stack is a test of the lane path's bound)
-        const bool few = work.stackCap == 0 && n <= kFewRays * ((gridDim.x * blockDim.x) >> 5);
+        const bool few = work.stackCap == 0 && n <= Work::kFewRays * ((gridDim.x * blockDim.x) >> 5);
         if (few && blockIdx.x * (blockDim.x >> 5) >= n) return;
         phase_begin(ctr, Work::kPhase);
         if (!few)
@@ -2803,12 +2808,13 @@ namespace pt
             batch_end_kernel<<<1, 1, 0, s>>>(b);
             return cudaGetLastError();
         }
-        // The frame's default variant and thresholds. Batches used the kernel with unconstrained registers (95, 5
-        // blocks per SM) and refilled a warp only when all 32 lanes were idle, so a warp ran until its longest
-        // ray ended: 2,097,153 any-hit rays on spheres-1m took 573 instead of 328 us, 262,147 closest-hit rays
-        // on spheres-200k 117 instead of 95 us.
+        // The frame's variant. Batches used the kernel with unconstrained registers (95, 5 blocks per SM) and refilled
+        // a warp only when all 32 lanes were idle, so a warp ran until its longest ray ended: 2,097,153 any-hit rays
+        // on spheres-1m took 573 instead of 328 us, 262,147 closest-hit rays on spheres-200k 117 instead of 95 us.
+        // Closest-hit warps refill at 12 idle lanes: at 4, 8, 12, 16 and 20, 2,097,153 rays on spheres-1m took 358,
+        // 354, 357, 371 and 397 us and on spheres-200k 202, 202, 199, 200 and 208 us; small batches the same.
         if (occOut) return launch_trace<true>(b, sc.depth, kBatchOccupancy, blocks, threads, 8, errorFlags, s);
-        return launch_trace<false>(b, sc.depth, kBatchOccupancy, blocks, threads, 16, errorFlags, s);
+        return launch_trace<false>(b, sc.depth, kBatchOccupancy, blocks, threads, 12, errorFlags, s);
     }
 }
 

@@ -16,9 +16,9 @@ def ray_mix(scene, n):
     return rays
 
 
-# 9 resident blocks of 4 warps on each of 148 multiprocessors, 4 rays per warp: 21,312 is the last size of the first kind
+# 9 resident blocks of 4 warps on each of 148 multiprocessors, 8 rays per warp: 42,624 is the last size of the first kind
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [1, 2, 33, 5329, 21312, 21313])
+@pytest.mark.parametrize("n", [1, 2, 33, 5329, 21313, 42624, 42625])
 @pytest.mark.parametrize("name", ["cornell", "cornell-all", "spheres-10k", "spheres-200k"])
 def test_batches_equal_the_binary_bvh(gpu_renderer, scene_factory, name, n):
     s = scene_factory(name)
@@ -45,7 +45,7 @@ def test_batches_of_several_threads(gpu_renderer, scene_factory):
     r = gpu_renderer
     r.upload_scene(s)
     batches = []
-    for n in (1, 700, 30001):
+    for n in (1, 700, 60001):
         rays = ray_mix(s, n)
         batches.append((torch.from_numpy(rays).cuda(),) + r.trace_closest_np(rays))
     torch.cuda.synchronize()

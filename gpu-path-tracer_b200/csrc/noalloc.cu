@@ -96,6 +96,9 @@ extern "C" int gpt_build_alias_table_noalloc(const float* weights, uint32_t ligh
     float* stackValue = reinterpret_cast<float*>(scratch + kStackValueOff);
     double* scan = reinterpret_cast<double*>(scratch + kScanOff);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (light_count <= pt::kAliasOneLaunch)
+        return pt::launch_alias_build_small(weights, light_count, reinterpret_cast<uint4*>(bins), stackIndex, stackValue, s) == cudaSuccess ? GPT_OK
+                                                                                                                                           : GPT_ERR_CUDA;
     const uint32_t blocks = (light_count + 255) / 256;
     weights_to_double_kernel<<<blocks, 256, 0, s>>>(weights, light_count, w);
     if (cudaGetLastError() != cudaSuccess) return GPT_ERR_CUDA;

@@ -148,9 +148,10 @@ namespace pt
     // check the decisions against the sums and write the bins. Steps from the first wrong prediction on are
     // discarded; one step (or kAliasSerial, if the window failed early) is taken by decision, and the next
     // window starts behind it. The bins are the sequential pairing's bits.
-    // Bound by the chain, about 10 cycles a step. gpt_build_alias_table_noalloc of 4,096 lights: 68 us, of
-    // 65,536 lights 0.85 ms; with one thread doing everything against global memory 735 us and 13.9 ms, with one
-    // thread pairing from shared memory 210 us and 3.1 ms.
+    // Bound by the chain and the synchronisations around it. gpt_build_alias_table_noalloc of 4,096 lights: 48 us, of
+    // 65,536 lights 0.67 ms (68 us and 0.85 ms before the chain read its values a group ahead and, up to
+    // kAliasOneLaunch lights, before the sum was formed here); with one thread doing everything against global memory
+    // 735 us and 13.9 ms, with one thread pairing from shared memory 210 us and 3.1 ms.
     constexpr uint32_t kAliasBlock = 1024;   // threads, and steps predicted at once
     constexpr uint32_t kAliasSerial = 256;
 
@@ -181,18 +182,55 @@ namespace pt
         return v;
     }
 
-    __global__ void __launch_bounds__(kAliasBlock) alias_build_kernel(const double* weights, const double* prefix, uint32_t n, uint4* bins,
+    // The weights' sum as exclusive_scan gives it, by one block: the scan's order of additions, for at most
+    // kAliasOneLaunch weights.
+    template <class T>
+    __device__ double alias_weight_sum(const T* weights, uint32_t n, double* warpSums)
+    {
+        __shared__ double chunkSums[kAliasOneLaunch / kAliasBlock], lastExclusive, offset;
+        const uint32_t chunks = (n + kAliasBlock - 1u) / kAliasBlock;
+        for (uint32_t c = 0; c < chunks; c++)
+        {
+            const uint32_t i = c * kAliasBlock + threadIdx.x;
+            const double x = i < n ? static_cast<double>(weights[i]) : 0.0;
+            const double inclusive = block_inclusive_sum(x, warpSums);
+            if (threadIdx.x == kAliasBlock - 1u) chunkSums[c] = inclusive;
+            if (i == n - 1u) lastExclusive = inclusive - x;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32)
+        {
+            const uint32_t lane = threadIdx.x;
+            const double x = lane < chunks ? chunkSums[lane] : 0.0;
+            double v = x;
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const double y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+                if (lane >= static_cast<uint32_t>(o)) v = v + y;
+            }
+            if (lane == chunks - 1u) offset = v - x;
+        }
+        __syncthreads();
+        const double last = chunks > 1u ? lastExclusive + offset : lastExclusive;
+        return last + static_cast<double>(weights[n - 1]);
+    }
+
+    // ONE: the sum of the weights is formed here (prefix is not read).
+    template <class T, bool ONE>
+    __global__ void __launch_bounds__(kAliasBlock) alias_build_kernel(const T* weights, const double* prefix, uint32_t n, uint4* bins,
                                                                       uint32_t* stackIndex, float* stackValue)
     {
         constexpr uint32_t W = kAliasBlock;
         __shared__ uint32_t underIndex[W], overIndex[W];
         __shared__ float underValue[W], overValue[W];
         __shared__ double underKey[W + 1], overKey[W + 1], warpSums[32];
-        __shared__ alignas(16) float stepValue[W], stepExcess[W + 4];
+        __shared__ alignas(16) float stepValue[W + 4], stepExcess[W + 4];
         __shared__ uint32_t warpUnder[32], steps, wrong, takenUnder, takenOver, liveShared;
         __shared__ float excessShared;
         const uint32_t lane = scan_lane_id(), warp = threadIdx.x >> 5, tid = threadIdx.x;
-        const float sum = static_cast<float>(prefix[n - 1] + weights[n - 1]);
+        float sum;
+        if constexpr (ONE) sum = static_cast<float>(alias_weight_sum(weights, n, warpSums));
+        else sum = static_cast<float>(prefix[n - 1] + weights[n - 1]);
         uint32_t* const overStackIndex = stackIndex + n;
         float* const overStackValue = stackValue + n;
         // classification, both lists in order
@@ -300,9 +338,11 @@ namespace pt
             {
                 // the chain; whole groups of 4, what lies behind the predicted steps is not used
                 float e = excess;
+                float4 next = *reinterpret_cast<const float4*>(stepValue);
                 for (uint32_t k = 0; k < predicted; k += 4)
                 {
-                    const float4 v = *reinterpret_cast<const float4*>(stepValue + k);
+                    const float4 v = next;
+                    next = *reinterpret_cast<const float4*>(stepValue + k + 4);
                     const float e1 = v.x + e - 1, e2 = v.y + e1 - 1, e3 = v.z + e2 - 1;
                     *reinterpret_cast<float4*>(stepExcess + k) = make_float4(e, e1, e2, e3);
                     e = v.w + e3 - 1;
@@ -637,9 +677,22 @@ namespace pt
                                    uint32_t* stackIndex, float* stackValue, cudaStream_t s)
     {
         if (n == 0) return cudaSuccess;
-        cudaError_t e = exclusive_scan<double>(weights, prefix, n, scanScratch, s);
-        if (e != cudaSuccess) return e;
-        alias_build_kernel<<<1, kAliasBlock, 0, s>>>(weights, prefix, n, bins, stackIndex, stackValue);
+        if (n <= kAliasOneLaunch)
+            alias_build_kernel<double, true><<<1, kAliasBlock, 0, s>>>(weights, nullptr, n, bins, stackIndex, stackValue);
+        else
+        {
+            const cudaError_t e = exclusive_scan<double>(weights, prefix, n, scanScratch, s);
+            if (e != cudaSuccess) return e;
+            alias_build_kernel<double, false><<<1, kAliasBlock, 0, s>>>(weights, prefix, n, bins, stackIndex, stackValue);
+        }
+        return cudaGetLastError();
+    }
+
+    cudaError_t launch_alias_build_small(const float* weights, uint32_t n, uint4* bins, uint32_t* stackIndex, float* stackValue, cudaStream_t s)
+    {
+        if (n == 0) return cudaSuccess;
+        if (n > kAliasOneLaunch) return cudaErrorInvalidValue;
+        alias_build_kernel<float, true><<<1, kAliasBlock, 0, s>>>(weights, nullptr, n, bins, stackIndex, stackValue);
         return cudaGetLastError();
     }
 

@@ -53,7 +53,7 @@ def weights_of(kind, n):
 # float weights of these sizes sum to the same float from any FP64 order
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["spread", "equal", "one", "halves", "thirds", "uniform"])
-@pytest.mark.parametrize("n", [1, 2, 31, 1023, 1024, 1025, 2047, 2048, 2049, 4096, 6145, 65536])
+@pytest.mark.parametrize("n", [1, 2, 31, 1023, 1024, 1025, 2047, 2048, 2049, 4096, 6145, 8192, 8193, 65536])
 def test_alias_table_equals_the_sequential_pairing(kind, n):
     import torch
     w = weights_of(kind, n)

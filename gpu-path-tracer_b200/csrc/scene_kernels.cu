@@ -148,8 +148,8 @@ namespace pt
     // check the decisions against the sums and write the bins. Steps from the first wrong prediction on are
     // discarded; one step (or kAliasSerial, if the window failed early) is taken by decision, and the next
     // window starts behind it. The bins are the sequential pairing's bits.
-    // Bound by the chain and the synchronisations around it. gpt_build_alias_table_noalloc of 4,096 lights: 48 us, of
-    // 65,536 lights 0.67 ms (68 us and 0.85 ms before the chain read its values a group ahead and, up to
+    // Bound by the chain and the synchronisations around it. gpt_build_alias_table_noalloc of 4,096 lights: 46 us, of
+    // 65,536 lights 0.65 ms (68 us and 0.85 ms before the chain read its values a group ahead and, up to
     // kAliasOneLaunch lights, before the sum was formed here); with one thread doing everything against global memory
     // 735 us and 13.9 ms, with one thread pairing from shared memory 210 us and 3.1 ms.
     constexpr uint32_t kAliasBlock = 1024;   // threads, and steps predicted at once
@@ -180,6 +180,43 @@ namespace pt
         if (warp > 0) v = v + warpSums[warp - 1];
         __syncthreads();
         return v;
+    }
+
+    // Two of them at once, with the synchronisations of one (4,096 lights 47.5 -> 45.5 us, 65,536 lights 670 -> 654 us).
+    __device__ void block_inclusive_sums(double& a, double& b, double* warpSums)
+    {
+        const uint32_t lane = scan_lane_id(), warp = threadIdx.x >> 5;
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const double x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_up_sync(0xFFFFFFFFu, b, o);
+            if (lane >= static_cast<uint32_t>(o))
+            {
+                a = a + x;
+                b = b + y;
+            }
+        }
+        if (lane == 31)
+        {
+            warpSums[warp] = a;
+            warpSums[32 + warp] = b;
+        }
+        __syncthreads();
+        if (warp < 2)
+        {
+            double w = warpSums[threadIdx.x];
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const double y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+                if (lane >= static_cast<uint32_t>(o)) w = w + y;
+            }
+            warpSums[threadIdx.x] = w;
+        }
+        __syncthreads();
+        if (warp > 0)
+        {
+            a = a + warpSums[warp - 1];
+            b = b + warpSums[31 + warp];
+        }
     }
 
     // The weights' sum as exclusive_scan gives it, by one block: the scan's order of additions, for at most
@@ -223,7 +260,7 @@ namespace pt
         constexpr uint32_t W = kAliasBlock;
         __shared__ uint32_t underIndex[W], overIndex[W];
         __shared__ float underValue[W], overValue[W];
-        __shared__ double underKey[W + 1], overKey[W + 1], warpSums[32];
+        __shared__ double underKey[W + 1], overKey[W + 1], warpSums[64];
         __shared__ alignas(16) float stepValue[W + 4], stepExcess[W + 4];
         __shared__ uint32_t warpUnder[32], steps, wrong, takenUnder, takenOver, liveShared;
         __shared__ float excessShared;
@@ -303,10 +340,9 @@ namespace pt
             // keys: under outcome i is taken before over outcome j if the excess with i unders and j overs taken,
             // excess0 - deficit(i) + surplus(j), is 1 or more; entry haveUnder (haveOver) is the end of the list
             const double start = static_cast<double>(excess) - 1.0;
-            const double deficits = block_inclusive_sum(deficit, warpSums);
-            const double surpluses = block_inclusive_sum(surplus, warpSums);
-            underKey[tid + 1] = deficits;
-            overKey[tid + 1] = start + surpluses;
+            block_inclusive_sums(deficit, surplus, warpSums);
+            underKey[tid + 1] = deficit;
+            overKey[tid + 1] = start + surplus;
             if (tid == 0)
             {
                 underKey[0] = 0.0;

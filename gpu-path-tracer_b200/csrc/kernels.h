@@ -94,7 +94,8 @@ namespace pt
     // 1,024 weights, instead of three to five launches before it (8,192 lights 120 -> 92 us, 1,024 lights 25 -> 16 us).
     // Above it the scan's blocks work side by side and the launches weigh less.
     constexpr uint32_t kAliasOneLaunch = 8192;
-    // launch_alias_build for at most kAliasOneLaunch float weights, without the prefix sums' scratch.
+    // launch_alias_build for at most kAliasOneLaunch float weights, without the prefix sums' scratch. The weights are read
+    // again while bins are written, so they have to lie outside the bins' memory.
     cudaError_t launch_alias_build_small(const float* weights, uint32_t n, uint4* bins, uint32_t* stackIndex, float* stackValue, cudaStream_t stream);
     cudaError_t launch_alias_build(const double* weights, uint32_t n, double* prefix, double* scanScratch, uint4* bins,
                                    uint32_t* stackIndex, float* stackValue, cudaStream_t stream);

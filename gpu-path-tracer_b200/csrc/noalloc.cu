@@ -96,7 +96,10 @@ extern "C" int gpt_build_alias_table_noalloc(const float* weights, uint32_t ligh
     float* stackValue = reinterpret_cast<float*>(scratch + kStackValueOff);
     double* scan = reinterpret_cast<double*>(scratch + kScanOff);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (light_count <= pt::kAliasOneLaunch)
+    // one launch reads the caller's weights while it writes bins; weights in the bins' memory are copied first, as large tables' are
+    const uintptr_t weightsAt = reinterpret_cast<uintptr_t>(weights), binsAt = reinterpret_cast<uintptr_t>(bins);
+    const bool apart = weightsAt + size_t(light_count) * 4 <= binsAt || binsAt + size_t(light_count) * 16 <= weightsAt;
+    if (light_count <= pt::kAliasOneLaunch && apart)
         return pt::launch_alias_build_small(weights, light_count, reinterpret_cast<uint4*>(bins), stackIndex, stackValue, s) == cudaSuccess ? GPT_OK
                                                                                                                                            : GPT_ERR_CUDA;
     const uint32_t blocks = (light_count + 255) / 256;

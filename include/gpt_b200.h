@@ -351,8 +351,9 @@ int gpt_bvh8_check(const gpt_scene_desc* scene, uint32_t* node_count, uint32_t* 
  * It builds the same table as the scene upload (AliasTable.hpp:22-84 semantics: FP64 sum of the
  * weights, p = w / sum, the reference's sequential pairing) from light_count float weights into
  * bins ([light_count][4] uint32 = q, p, alias, value). Both pointers are device memory; bins must be
- * 16-byte aligned and weights 4-byte aligned (GPT_ERR_INVALID_ARGUMENT otherwise). The weights must
- * be finite and non-negative with a positive sum; other weights give NaN or infinite entries.
+ * 16-byte aligned and weights 4-byte aligned (GPT_ERR_INVALID_ARGUMENT otherwise). The weights are
+ * read or copied before a bin is written over them, so they may lie anywhere in the bins' memory.
+ * They must be finite and non-negative with a positive sum; other weights give NaN or infinite entries.
  * light_count 0 returns GPT_OK and touches nothing. stream may be NULL (the legacy default
  * stream); the call is asynchronous on it.
  * Working memory is a fixed array of about 2 MiB compiled into the library, held by every GPU that

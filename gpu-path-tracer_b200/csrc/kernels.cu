@@ -2146,7 +2146,7 @@ namespace pt
     {
         __shared__ uint64_t endOf[kPlanJobs], launchedOf[kPlanJobs], totalOf[kPlanJobs];
         __shared__ uint32_t orderOf[kPlanJobs];
-        __shared__ bool activeOf[kPlanJobs], full;
+        __shared__ bool activeOf[kPlanJobs];
         EngineCtl* e = ev.ctl;
         const uint32_t avail = finished_paths(wf) + e->freeCount;
         const uint32_t orderCount = e->orderCount;
@@ -2154,8 +2154,7 @@ namespace pt
         // a job marked kOrderInTurn gets slots only once every marked job before it has launched all
         // its samples (its turn has come), even if an earlier one's pass window holds it back for now
         bool waitTurn = false;
-        if (threadIdx.x == 0) full = avail == 0;
-        for (uint32_t base = 0; base < orderCount; base += kPlanJobs)
+        for (uint32_t base = 0; avail != 0 && base < orderCount; base += kPlanJobs)
         {
             const uint32_t mine = base + threadIdx.x;
             if (mine < orderCount)
@@ -2169,7 +2168,6 @@ namespace pt
                 totalOf[threadIdx.x] = J.totalSamples;
             }
             __syncthreads();
-            if (full) break;
             if (threadIdx.x == 0)
             {
                 const uint32_t count = orderCount - base < kPlanJobs ? orderCount - base : kPlanJobs;
@@ -2192,9 +2190,9 @@ namespace pt
                     }
                     if (inTurn && launched < totalOf[i]) waitTurn = true;
                 }
-                full = launch >= avail;
             }
-            __syncthreads();
+            // all threads leave together once the slots have run out
+            if (__syncthreads_or(threadIdx.x == 0 && launch >= avail)) break;
         }
         if (threadIdx.x != 0) return;
         e->launchCount = launch;

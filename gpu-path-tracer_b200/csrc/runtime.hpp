@@ -207,7 +207,9 @@ namespace pt
             if (bytes >= (ready_ ? kSmallest : kSmallestFirst))
             {
                 job.lock_ = std::unique_lock<std::mutex>(mutex_);
-                if (prepare())
+                if (!prepare())
+                    cudaGetLastError();  // copied without it; a later launch must not report this error as its own
+                else
                 {
                     job.items_ = std::move(items);
                     job.next_ = 0;
@@ -243,7 +245,6 @@ namespace pt
             if (!pinned_ && cudaHostAlloc(&pinned_, kLanes * kSlots * kChunk, cudaHostAllocPortable) != cudaSuccess)
             {
                 pinned_ = nullptr;
-                cudaGetLastError();  // copied without it
                 return false;
             }
             for (int k = 0; k < kLanes; k++)

@@ -345,14 +345,13 @@ namespace pt
             }
             PT_CUDA("cudaEventCreate", cudaEventCreate(&startEvent_));
             PT_CUDA("cudaEventCreate", cudaEventCreate(&stopEvent_));
-            PT_CUDA("cudaHostAlloc", cudaHostAlloc(&hostMapped_, 64 + 4 * kBatchStates, cudaHostAllocMapped));
-            std::memset(hostMapped_, 0, 64 + 4 * kBatchStates);
+            PT_CUDA("cudaHostAlloc", cudaHostAlloc(&hostMapped_, 64 + 4 * BatchStates::kCount, cudaHostAllocMapped));
+            std::memset(hostMapped_, 0, 64 + 4 * BatchStates::kCount);
             PT_CUDA("cudaHostGetDevicePointer", cudaHostGetDevicePointer(&hostMappedDev_, hostMapped_, 0));
             PT_TRY(job_.allocate(sizeof(JobView)));
             PT_TRY(counters_.allocate(sizeof(Counters)));
-            PT_TRY(batches_.allocate(kBatchStates * sizeof(BatchState)));
-            PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(batches_.get<void>(), 0, kBatchStates * sizeof(BatchState), stream_));
-            PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream_));
+            PT_TRY(batches_.create(reinterpret_cast<volatile uint32_t*>(static_cast<char*>(hostMapped_) + 64),
+                                   reinterpret_cast<uint32_t*>(static_cast<char*>(hostMappedDev_) + 64), stream_));
             return Status::Ok();
         }
 
@@ -844,39 +843,10 @@ namespace pt
             const SceneView sv = scene_->view();
             if (bvh == kBvh2Fp32 && !sv.nodes2) return Status::Err(GPT_ERR_STATE, "The scene has no binary BVH");
             const int blocks = trace_grid_blocks(device_, 128, sv.depth, kBatchOccupancy, bvh);
-            const BatchSlot slot(*this);
-            volatile uint32_t* errors = reinterpret_cast<volatile uint32_t*>(static_cast<char*>(hostMapped_) + 64) + slot.index;
-            uint32_t* errorsDev = reinterpret_cast<uint32_t*>(static_cast<char*>(hostMappedDev_) + 64) + slot.index;
-            *errors = 0u;
-            PT_CUDA("intersect", launch_batch_trace(sv, 0u, rays, n, batches_.get<BatchState>() + slot.index, errorsDev, tri, uvt, occ, blocks, 128, st, bvh));
-            PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(st));
-            if (*errors) return Status::Err(GPT_ERR_DEVICE_FAULT, "Traversal reported error flags " + std::to_string(*errors));
-            return Status::Ok();
+            BatchStates::Call call(batches_);
+            PT_TRY(call.begin(st));
+            return call.end(launch_batch_trace(sv, 0u, rays, n, call.state(), call.errorsDevice(), tri, uvt, occ, blocks, 128, st, bvh), st);
         }
-
-        // One of the batch states, for one call: callers on several threads get different ones.
-        struct BatchSlot
-        {
-            Renderer& impl;
-            uint32_t index;
-            explicit BatchSlot(Renderer& i) : impl(i)
-            {
-                std::unique_lock lock(impl.batchMutex_);
-                impl.batchFreed_.wait(lock, [&] { return impl.batchesFree_ != 0; });
-                index = static_cast<uint32_t>(__builtin_ctz(impl.batchesFree_));
-                impl.batchesFree_ &= impl.batchesFree_ - 1u;
-            }
-            ~BatchSlot()
-            {
-                {
-                    std::scoped_lock lock(impl.batchMutex_);
-                    impl.batchesFree_ |= 1u << index;
-                }
-                impl.batchFreed_.notify_one();
-            }
-            BatchSlot(const BatchSlot&) = delete;
-            BatchSlot& operator=(const BatchSlot&) = delete;
-        };
 
         // ---------------------------------------------------------------- simulation thread
         Status StartSimulation(uint32_t width, uint32_t height, float fovY, const gpt_motion_state* states, uint32_t count, uint32_t spp,
@@ -1014,15 +984,12 @@ namespace pt
         cudaStream_t shadeStreams_[kModelCount] = {};
         void* hostMapped_ = nullptr;
         void* hostMappedDev_ = nullptr;  // [0] cancel flag, [16] progress, [32] loop condition, [64] error flags of the batch states
-        static constexpr uint32_t kBatchStates = 16;
-        std::mutex batchMutex_;
-        std::condition_variable batchFreed_;
-        uint32_t batchesFree_ = (1u << kBatchStates) - 1u;
+        BatchStates batches_;
         static constexpr uint32_t kDefaultPool = 1u << 20;
         static constexpr uint32_t kLogCapacity = 1u << 16;
         uint32_t pool_ = 0;
         DeviceBuffer rays_[2], matQ_, shRays_, shL_, regen_, regenBits_, slots_, slotSample_, queueLog_;
-        DeviceBuffer counters_, job_, batches_, accumulation_, framebuffer_, sampleRadiance_;
+        DeviceBuffer counters_, job_, accumulation_, framebuffer_, sampleRadiance_;
         JobView hostJob_{};
         Counters hostCounters_{};
         std::unique_ptr<SceneGpu> scene_;

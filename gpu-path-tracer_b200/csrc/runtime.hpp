@@ -5,6 +5,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <atomic>
+#include <condition_variable>
 #include <cstdint>
 #include <cstring>
 #include <memory>
@@ -15,6 +16,7 @@
 #include <vector>
 
 #include "../../include/gpt_b200.h"
+#include "kernels.h"
 #include "pt_internal.h"
 
 namespace pt
@@ -31,6 +33,7 @@ namespace pt
     inline Status CudaStatus(const char* op, cudaError_t e)
     {
         if (e == cudaSuccess) return Status::Ok();
+        cudaGetLastError();  // reported here; left as the thread's last error, the next launch would report it as its own
         // Error text format of the reference (Cuda/Utils/Error.cpp:22-25).
         std::string msg = std::string(op) + " failed: " + cudaGetErrorName(e) + ": " + cudaGetErrorString(e);
         return Status::Err(e == cudaErrorMemoryAllocation ? GPT_ERR_OUT_OF_MEMORY : GPT_ERR_CUDA, msg);
@@ -292,6 +295,85 @@ namespace pt
         void* pinned_ = nullptr;
         Lane lanes_[kLanes];
         std::atomic<bool> ready_{false};
+    };
+
+    // The states of a renderer's ray batches, one for each call in flight: callers on several threads get different ones,
+    // and a call beyond kCount waits for one of them. A batch's last block leaves its state all zero. A call that failed
+    // between its launches may have left something in it, so a state whose last call did not end well is cleared before
+    // the next one's launch.
+    class BatchStates
+    {
+    public:
+        static constexpr uint32_t kCount = 16;
+
+        // errors, errorsDevice: a host-mapped word per state.
+        Status create(volatile uint32_t* errors, uint32_t* errorsDevice, cudaStream_t stream)
+        {
+            errors_ = errors;
+            errorsDevice_ = errorsDevice;
+            PT_TRY(states_.allocate(kCount * sizeof(BatchState)));
+            PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(states_.get<void>(), 0, kCount * sizeof(BatchState), stream));
+            PT_CUDA("cudaStreamSynchronize", cudaStreamSynchronize(stream));
+            return Status::Ok();
+        }
+
+        // One call: begin(), the launches, end().
+        class Call
+        {
+        public:
+            explicit Call(BatchStates& all) : all_(all)
+            {
+                std::unique_lock lock(all_.mutex_);
+                all_.freed_.wait(lock, [&] { return all_.free_ != 0; });
+                index_ = static_cast<uint32_t>(__builtin_ctz(all_.free_));
+                all_.free_ &= all_.free_ - 1u;
+            }
+            ~Call()
+            {
+                {
+                    std::scoped_lock lock(all_.mutex_);
+                    all_.free_ |= 1u << index_;
+                }
+                all_.freed_.notify_one();
+            }
+            Call(const Call&) = delete;
+            Call& operator=(const Call&) = delete;
+
+            BatchState* state() const { return all_.states_.get<BatchState>() + index_; }
+            uint32_t* errorsDevice() const { return all_.errorsDevice_ + index_; }
+
+            Status begin(cudaStream_t stream)
+            {
+                all_.errors_[index_] = 0u;
+                if (all_.unclean_[index_]) PT_CUDA("cudaMemsetAsync", cudaMemsetAsync(state(), 0, sizeof(BatchState), stream));
+                all_.unclean_[index_] = true;
+                return Status::Ok();
+            }
+            // Waits for what was launched, whether or not all of it was.
+            Status end(cudaError_t launched, cudaStream_t stream)
+            {
+                const cudaError_t done = cudaStreamSynchronize(stream);
+                PT_CUDA("intersect", launched);
+                PT_CUDA("cudaStreamSynchronize", done);
+                all_.unclean_[index_] = false;
+                const uint32_t errors = all_.errors_[index_];
+                if (errors) return Status::Err(GPT_ERR_DEVICE_FAULT, "Traversal reported error flags " + std::to_string(errors));
+                return Status::Ok();
+            }
+
+        private:
+            BatchStates& all_;
+            uint32_t index_;
+        };
+
+    private:
+        DeviceBuffer states_;
+        volatile uint32_t* errors_ = nullptr;
+        uint32_t* errorsDevice_ = nullptr;
+        std::mutex mutex_;
+        std::condition_variable freed_;
+        uint32_t free_ = (1u << kCount) - 1u;
+        bool unclean_[kCount] = {};  // (only the call that holds a state touches its entry)
     };
 
     // An image texture with the reference's descriptors (Texture.cpp:65-189).

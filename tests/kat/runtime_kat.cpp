@@ -13,7 +13,7 @@ namespace
 {
     std::string g_failing;         // name of the call that fails
     std::atomic<int> g_before{0};  // how many of these calls succeed first
-    std::atomic<int> g_streamCopies{0}, g_laneCopies{0};
+    std::atomic<int> g_streamCopies{0}, g_laneCopies{0}, g_memsets{0};
     thread_local cudaError_t t_last = cudaSuccess;
     int g_wrong = 0;
     const cudaStream_t kCallersStream = reinterpret_cast<cudaStream_t>(1);
@@ -57,6 +57,12 @@ extern "C"
     }
     cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
     cudaError_t cudaStreamSynchronize(cudaStream_t) { return result("cudaStreamSynchronize", cudaErrorStreamCaptureUnsupported); }
+    cudaError_t cudaMemsetAsync(void* p, int value, size_t n, cudaStream_t)
+    {
+        g_memsets++;
+        std::memset(p, value, n);
+        return cudaSuccess;
+    }
     cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
     {
         const cudaError_t r = result("cudaEventCreateWithFlags", cudaErrorMemoryAllocation);
@@ -123,6 +129,50 @@ namespace
         upload(through, 2u);
         expect(g_streamCopies == 0 && g_laneCopies > 0, "pinned copies once they can be had");
     }
+
+    // A batch that took `rays` rays; it leaves its state clear unless its last launch was not made.
+    pt::Status batch(pt::BatchStates& states, uint32_t rays, cudaError_t launched)
+    {
+        pt::BatchStates::Call call(states);
+        const pt::Status begun = call.begin(kCallersStream);
+        if (!begun.ok()) return begun;
+        pt::BatchState* s = call.state();
+        expect(s->cursor == 0 && s->errors == 0 && s->left == 0, "a batch starts from a clear state");
+        s->cursor = rays;
+        if (launched == cudaSuccess) *s = pt::BatchState{};
+        return call.end(launched, kCallersStream);
+    }
+
+    void batches(cudaError_t launched, const char* failing)
+    {
+        uint32_t errors[pt::BatchStates::kCount] = {};
+        pt::BatchStates states;
+        expect(states.create(errors, errors, kCallersStream).ok(), "the states");
+        g_memsets = 0;
+        for (uint32_t k = 0; k < 3; k++) expect(batch(states, 100u, cudaSuccess).ok(), "a batch");
+        expect(g_memsets == 0, "batches that ended well are not cleared again");
+        g_failing = failing;
+        expect(!batch(states, 100u, launched).ok(), "the failure is reported");
+        expect(cudaGetLastError() == cudaSuccess, "no error is left for the next launch");
+        g_failing.clear();
+        for (uint32_t k = 0; k < 3; k++) expect(batch(states, 100u, cudaSuccess).ok(), "a batch behind the failure");
+        expect(g_memsets == 1, "cleared once");
+        // as many failures as there are states use none of them up
+        for (uint32_t k = 0; k < 2 * pt::BatchStates::kCount; k++) expect(!batch(states, 7u, cudaErrorLaunchOutOfResources).ok(), "the failure is reported");
+        expect(batch(states, 100u, cudaSuccess).ok(), "a batch behind many failures");
+    }
+
+    // Callers on more threads than there are states: each has a state to itself.
+    void batches_of_threads()
+    {
+        uint32_t errors[pt::BatchStates::kCount] = {};
+        pt::BatchStates states;
+        expect(states.create(errors, errors, kCallersStream).ok(), "the states");
+        std::vector<std::thread> callers;
+        for (uint32_t t = 0; t < 2 * pt::BatchStates::kCount; t++)
+            callers.emplace_back([&states, t] { for (uint32_t k = 0; k < 200; k++) batch(states, t + 1u, k % 5 ? cudaSuccess : cudaErrorLaunchOutOfResources); });
+        for (std::thread& t : callers) t.join();
+    }
 }
 
 int main(int argc, char** argv)
@@ -155,6 +205,12 @@ int main(int argc, char** argv)
         g_failing.clear();
         upload(through, 2u);
     }
+    else if (name == "a batch whose second launch fails")
+        batches(cudaErrorLaunchOutOfResources, "");
+    else if (name == "a batch that cannot be waited for")
+        batches(cudaSuccess, "cudaStreamSynchronize");
+    else if (name == "batches of many threads")
+        batches_of_threads();
     else if (name == "two uploads at once")
     {
         pt::PinnedUpload through;

@@ -19,7 +19,8 @@ def runtime_kat(tmp_path_factory):
 
 @pytest.mark.parametrize("case", [
     "upload", "upload without pinned memory", "upload without streams", "upload without the last stream",
-    "upload without events", "upload without threads", "upload with two threads", "upload that fails", "two uploads at once"])
+    "upload without events", "upload without threads", "upload with two threads", "upload that fails", "two uploads at once",
+    "a batch whose second launch fails", "a batch that cannot be waited for", "batches of many threads"])
 def test_runtime_with_failing_calls(runtime_kat, case):
     p = subprocess.run([runtime_kat, case], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, p.stdout + p.stderr

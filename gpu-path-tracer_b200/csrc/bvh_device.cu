@@ -598,7 +598,7 @@ namespace pt
                     slotUsed[bs] = true;
                     slotOf[bk] = bs;
                 }
-                // child references: inner children take consecutive indices in the order of the child list
+                // the children's block; inner children take consecutive indices in the order of the child list
                 int inner = 0;
                 for (int i = 0; i < nk; i++) inner += kidLeaf[i] ? 0 : 1;
                 const uint32_t firstInner = inner ? atomicAdd(counter, static_cast<uint32_t>(inner)) : 0u;

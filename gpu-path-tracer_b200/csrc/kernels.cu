@@ -510,7 +510,8 @@ namespace pt
     // Persistent traversal: each warp keeps 32 rays in flight; when at least `refill` lanes are
     // idle the warp takes that many new rays with one atomic (ballot + popc + shuffle), so lanes
     // that finished early are refilled instead of idling until the slowest ray of the warp ends.
-    // The plain format: the binary FP32 BVH with a per-thread stack of kMaxStack entries in local memory.
+    // The plain format: the binary FP32 BVH with a per-thread stack of kMaxStack entries in local memory, a node's
+    // nearer child first.
     // Shared memory: [cold slots: 2 x float4 per thread].
     template <bool ANY, class Work>
     __global__ void __launch_bounds__(128, 1) trace_binary_kernel(Work work, uint32_t refill, uint32_t* errorFlags)
@@ -553,11 +554,6 @@ namespace pt
                         cold.p[0] = make_float4(d.x, d.y, d.z, __uint_as_float(tag));
                         cold.p[1] = make_float4(0.0f, 0.0f, __uint_as_float(kInvalid), __uint_as_float(i));
                         st.ray = make_ray(o, d, tmin);
-                        // Any-hit rays visit a node's children far to near (from the light's end of the
-                        // segment): the first occluder found ends the ray, and occluders lie nearer the
-                        // light more often than near the shaded point (8.19M-triangle scene: 12.2 instead
-                        // of 15.0 node visits per shadow ray). The order changes no result.
-                        if (ANY) st.ray.oct ^= 7u;
                         st.hitT = tmax;
                         st.pending = work.root(tag);
                         st.sp = 0;
@@ -759,7 +755,8 @@ namespace pt
         }
     }
 
-    // The same for the BVH8, with the warp's lanes in step: each step visits a few nodes per lane, then tests
+    // Persistent traversal of the BVH8, refilled as in trace_binary_kernel, or a warp per ray (trace_few) when there
+    // are few rays. The warp's lanes are in step: each step visits a few nodes per lane, then tests
     // one triangle per lane if enough lanes hold leaves (kLeafShare), and goes on testing while more than
     // half of the busy lanes do. A node visit rarely enters leaves in more than a few lanes (0.34 tests per
     // visit on spheres-1m), so testing them at once ran the triangle test for 7, then 2, then 1 lane of the
@@ -857,6 +854,10 @@ namespace pt
                             cold.p[0] = make_float4(d.x, d.y, d.z, __uint_as_float(tag));
                             cold.p[1] = make_float4(0.0f, 0.0f, __uint_as_float(kInvalid), __uint_as_float(i));
                             st.ray = make_ray(o, d, tmin);
+                            // Any-hit rays visit a node's children far to near (from the light's end of the
+                            // segment): the first occluder found ends the ray, and occluders lie nearer the
+                            // light more often than near the shaded point (8.19M-triangle scene: 12.2 instead
+                            // of 15.0 node visits per shadow ray). The order changes no result.
                             if (ANY) st.ray.oct ^= 7u;
                             st.hitT = tmax;
                             stack[0] = (work.root(tag) << 8) | (1u << st.ray.oct);
@@ -2786,7 +2787,8 @@ namespace pt
         }
         // The frame's variant. Batches used the kernel with unconstrained registers (95, 5 blocks per SM) and refilled
         // a warp only when all 32 lanes were idle, so a warp ran until its longest ray ended: 2,097,153 any-hit rays
-        // on spheres-1m took 573 instead of 328 us, 262,147 closest-hit rays on spheres-200k 117 instead of 95 us.
+        // on spheres-1m took 573 instead of 328 us, 262,147 closest-hit rays on spheres-200k 117 instead of 95 us (with
+        // the kernels of today 251 and 82 us).
         // Closest-hit warps refill at 12 idle lanes: at 4, 8, 12, 16 and 20, 2,097,153 rays on spheres-1m took 358,
         // 354, 357, 371 and 397 us and on spheres-200k 202, 202, 199, 200 and 208 us; small batches the same.
         if (occOut) return launch_trace<true>(b, sc.depth, kBatchOccupancy, blocks, threads, 8, errorFlags, s);

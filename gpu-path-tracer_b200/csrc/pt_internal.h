@@ -62,8 +62,8 @@ namespace pt
     // reference in another sector of the node.
     //  Node header:
     //   w[0] = qx << 8 | inner mask, qy << 8 | u, qz << 8 | ez[2:0] << 5 | ex, block << 8 | ez[4:3] << 5 | ey
-    //          origin = q * 2^(u - 119) per axis (q signed, 24 bits: the float precision of its largest
-    //          coordinate), box scale of an axis = 2^(u - 126 + e), block = the node's child block
+    //          origin = q * 2^(u - 119) per axis (q signed, |q| < 2^23: a bit less than the float precision of
+    //          its largest coordinate), box scale of an axis = 2^(u - 126 + e), block = the node's child block
     //   w[1] = qlo.x[0..7] (x,y words), qlo.y[0..7] (z,w words)
     //   w[2] = qlo.z[0..7], qhi.x[0..7]
     //   w[3] = qhi.y[0..7], qhi.z[0..7]

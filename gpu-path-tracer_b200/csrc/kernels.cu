@@ -1930,10 +1930,12 @@ namespace pt
         return k;
     }
 
-    // Phase times into their sums, and the counters' values for the next iteration. Called by one warp.
+    // Phase times into their sums, and the counters' values for the next iteration. Called by one warp, whose lanes have
+    // all read the current values (the shuffles that passed them on order no memory).
     __device__ __forceinline__ void reset_iteration(Counters* c, const IterationCounts& k, uint32_t next)
     {
         const uint32_t lane = lane_id();
+        __syncwarp();
         if (lane < 4)
         {
             const unsigned long long start = c->tStart[lane].v, end = c->tEnd[lane].v;

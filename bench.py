@@ -759,10 +759,10 @@ def b200_arm(args):
         "scene_upload_s": upload_s,
         "scene_upload_breakdown_s": upload_breakdown,
         "traversal": traversal_summary(stats[-1], NODE_BYTES),
-        "roofline": {"kernel": "trace_kernel<closest> (BVH8 closest hit)", "bound": "latency", "achieved": achieved,
+        "roofline": {"kernel": "trace_kernel<closest> (BVH8 closest hit)", "bound": "issue", "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                      "dram_frac": (traffic / per_launch_s / 1e9 / peak) if traffic else None,
-                     "bound_note": "load latency and lane divergence: the algorithmic node/triangle bytes (frac) are served mostly "
+                     "bound_note": "instruction issue and lane divergence: the algorithmic node/triangle bytes (frac) are served mostly "
                                    "by L1/L2; dram_frac is the DRAM traffic of a launch over its duration against the same peak",
                      "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": per_launch_bytes,
